@@ -4,14 +4,12 @@ Drop-in for the reference operator (reference: src/bob/sdpa.py:387-468): same si
 exceptions raised before any launch (reference: src/bob/sdpa.py:21-137, pinned by
 tests/unit/test_attention_validation.py:14-56), same offset and window inference
 (reference: src/bob/sdpa.py:371-384, src/bob/attention.py:93-102) and the same autograd
-protocol (reference: src/bob/sdpa.py:239-368):
+protocol (reference: src/bob/sdpa.py:239-368), whose nodes are native (csrc/torch_binding.cpp):
 
-  * `SDPAWithBoB.forward` runs the forward kernel and keeps (q, k, v, out, lse);
-  * `SDPAWithBoB.backward` runs only the first backward when grad mode is off, otherwise it
-    applies `BoBSecondOrder`, whose forward is the first backward and whose backward is the
-    second backward returning gradients for (q, k, v, dO);
-  * undefined incoming tangents arrive as None (`set_materialize_grads(False)`) and switch off
-    the products they would feed.
+  * the forward runs the forward kernel and keeps (q, k, v, out, lse);
+  * its backward runs only the first backward when grad mode is off, otherwise it also records a
+    node over (q, k, v, dO) whose backward is the second backward, returning gradients for those;
+  * undefined incoming tangents stay undefined and switch off the products they would feed.
 
 CUDA tensors always go through the CUDA library: there is no fallback, a missing library raises.
 CPU tensors take PyTorch's math attention with stock autograd, exactly as the reference's CPU
@@ -25,9 +23,8 @@ import numbers
 import operator as _operator
 
 import torch
-from torch.autograd import Function
 
-from . import ops
+from . import _native, ops
 
 __all__ = ["sdpa_bob"]
 
@@ -162,66 +159,6 @@ def _cpu_math_attention(q, k, v, *, is_causal, window, q_offset, k_offset, scale
 
 
 # --------------------------------------------------------------------------------------
-# autograd chain
-# --------------------------------------------------------------------------------------
-class BoBSecondOrder(Function):
-    """First backward as a differentiable function of (q, k, v, dO); its backward is the
-    second backward (gradients for q, k, v and dO)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, dO, out, lse, q_offset, k_offset, is_causal, window_size, scale):
-        ctx.set_materialize_grads(False)
-        geom = dict(is_causal=is_causal, window_size=window_size, q_offset=q_offset,
-                    k_offset=k_offset, scale=scale)
-        dQ, dK, dV, delta, pk = ops.attention_first_backward(q, k, v, out, lse, dO, **geom)
-        ctx.save_for_backward(q, k, v, out, lse, dO, dQ, delta, pk)
-        ctx.geom = geom
-        return dQ, dK, dV
-
-    @staticmethod
-    def backward(ctx, uQ, uK, uV):
-        q, k, v, out, lse, dO, dQ, delta, pk = ctx.saved_tensors
-        if uQ is None and uK is None and uV is None:
-            return (None,) * 11
-        Qbar, Kbar, Vbar, dObar = ops.attention_second_backward(
-            q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV, **ctx.geom)
-        return (Qbar, Kbar, Vbar, dObar, None, None, None, None, None, None, None)
-
-
-class SDPAWithBoB(Function):
-    """Attention forward whose backward is itself differentiable once more."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, q_offset, k_offset, is_causal, window_size, scale):
-        # An undefined cotangent (the second differentiation of leaf-cotangent protocols reaches this
-        # node with nothing to propagate) must not be turned into a tensor of zeros and pushed
-        # through a pointless first backward.
-        ctx.set_materialize_grads(False)
-        q_offset = 0 if q_offset is None else int(q_offset)
-        k_offset = 0 if k_offset is None else int(k_offset)
-        geom = dict(is_causal=is_causal, window_size=window_size, q_offset=q_offset,
-                    k_offset=k_offset, scale=scale)
-        out, lse = ops.attention_forward(q, k, v, **geom)
-        ctx.save_for_backward(q, k, v, out, lse)
-        ctx.geom = geom
-        return out
-
-    @staticmethod
-    def backward(ctx, dO):
-        if dO is None:
-            return (None,) * 8
-        q, k, v, out, lse = ctx.saved_tensors
-        g = ctx.geom
-        if not torch.is_grad_enabled():
-            dQ, dK, dV, _, _ = ops.attention_first_backward(q, k, v, out, lse, dO,
-                                                            for_second_order=False, **g)
-        else:
-            dQ, dK, dV = BoBSecondOrder.apply(q, k, v, dO, out, lse, g["q_offset"], g["k_offset"],
-                                              g["is_causal"], g["window_size"], g["scale"])
-        return dQ, dK, dV, None, None, None, None, None
-
-
-# --------------------------------------------------------------------------------------
 # public operator
 # --------------------------------------------------------------------------------------
 def sdpa_bob(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, is_causal: bool = False,
@@ -239,6 +176,12 @@ def sdpa_bob(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, is_causal: bo
         raise NotImplementedError(
             "torch.func transforms are unsupported; differentiate with reverse mode "
             "(torch.autograd.grad twice) instead")
+    # The usual valid CUDA call is recognised natively (a few hundred nanoseconds); everything else comes
+    # back as None and takes the checks below.
+    if isinstance(q, torch.Tensor) and q.is_cuda:
+        out = _native.load().try_sdpa(q, k, v, is_causal, scale, window_size, q_offset, k_offset, ops._CHECK_STATUS)
+        if out is not None:
+            return out
     _check_tensors(q, k, v)
     window, q_off, k_off = _check_scalars(is_causal, scale, window_size, q_offset, k_offset)
     n_q, n_k = q.shape[2], k.shape[2]
@@ -257,4 +200,4 @@ def sdpa_bob(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, is_causal: bo
     if not q.is_cuda:
         return _cpu_math_attention(q, k, v, is_causal=is_causal, window=window, q_offset=q_off,
                                    k_offset=k_off, scale=scale, rectangular=rectangular)
-    return SDPAWithBoB.apply(q, k, v, q_off, k_off, is_causal, window, scale)
+    return _native.load().sdpa(q, k, v, is_causal, window, q_off, k_off, scale, ops._CHECK_STATUS)
