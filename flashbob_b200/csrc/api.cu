@@ -81,65 +81,41 @@ static int sm_count(int device) {
     return cache[device];
 }
 
-// Column-owned kernels: number of TN-wide query tiles that the 128 keys of own tile `own_tile` sweep
-// (the host's copy of the kernel's item decoding: same clipping of the causal / window range).
-static int col_sweep_tiles(const bob_sm100_geom* g, long long doff, int own_tile, int TN) {
-    const long long own0 = 128LL * own_tile, own_last = std::min<long long>(own0 + 127, g->Nk - 1);
-    long long lo = 0, hi = g->Nq;
-    if (g->is_causal) {
-        lo = std::max<long long>(0, own0 - doff);
-        if (g->window > 0) hi = std::min<long long>(g->Nq, own_last - doff + g->window);
-    }
-    if (hi <= lo) return 0;
-    return (int)((hi + TN - 1) / TN - lo / TN);
-}
-
-// Even split of a persistent column-owned launch over `ctas` CTAs: tile pairs per CTA, or 0 when the
-// split does not apply (too little work per CTA to pay for the cut items' extra epilogues, or a list
-// too long for 32-bit positions).
-static int even_split_span(const bob_sm100_geom* g, long long doff, int TN, int ctas) {
-#ifndef BOB_EVEN_SPLIT
-    // Off: measured slower than the counter-fed item queue (a span of equally many tile pairs holds very
-    // different numbers of items, and every item costs a prologue and an epilogue).
-    (void)g; (void)doff; (void)TN; (void)ctas;
-    return 0;
-#endif
-    const int n_own_tiles = (g->Nk + 127) / 128;
-    const long long per_rank = (long long)g->Hkv * g->B, G = g->Hq / g->Hkv;
-    long long total = 0;
-    for (int r = 0; r < n_own_tiles; ++r) total += (long long)col_sweep_tiles(g, doff, r, TN) * G * per_rank;
-    if (total <= 0 || total >= (1LL << 30)) return 0;
-    const long long span = (total + ctas - 1) / ctas;
-    return span >= 32 ? (int)span : 0;
-}
-
-static size_t even_split_flag_bytes(const bob_sm100_geom* g) {
-    return round256((size_t)((g->Nk + 127) / 128) * g->Hkv * g->B * sizeof(int));
-}
-static size_t even_split_park_bytes(int ctas) { return (size_t)ctas * 2 * 2 * 128 * 64 * sizeof(float); }
-
-// Whether a column-owned launch of this geometry is persistent (one CTA per SM taking many items).
-static bool col_launch_is_persistent(const bob_sm100_geom* g, int sms) {
-    return (long long)((g->Nk + 127) / 128) * g->Hkv * g->B > sms;
-}
-
 struct TensorArg {
     const void* ptr;
     const int64_t* strides;   // batch, head, row
     bool q_side;              // [B, Hq, Nq, D] (true) or [B, Hkv, Nk, D] (false)
 };
 
-template <int MODE, int DPAD, int TN, bool BF16, int NG = 1, int CW = 16>
+// Raises a kernel's shared-memory limit, once per device: the attribute calls are slow enough to show at
+// small sizes.
+template <class CFG, class Kernel>
+static int prepare_kernel(Kernel kernel, int device, std::atomic<uint64_t>& done) {
+    const uint64_t bit = 1ull << device;
+    if (done.load(std::memory_order_acquire) & bit) return 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM_BYTES) != cudaSuccess) return kErrAttr;
+    // The kernel's warpgroups trade registers after launch; the trade only balances (and the pointwise
+    // warps' request can only ever be met) if the kernel was built with the register count the trade
+    // assumes.  Refuse to launch otherwise.
+    cudaFuncAttributes a;
+    const int regs_at_launch = cudaFuncGetAttributes(&a, kernel) == cudaSuccess ? a.numRegs : 0;
+    if (regs_at_launch * CFG::NTHREADS < CFG::NPW * CFG::REGS_POINTWISE + 128 * CFG::REGS_ROLE) return kErrRegs;
+    done.fetch_or(bit, std::memory_order_release);
+    return 0;
+}
+
+template <int MODE, int DPAD, int TN, bool BF16, int NG, int CW, bool ALIAS>
 static int launch_sweep(const bob_sm100_geom* g, SweepParams& prm, const TensorArg* tensors,
                         cudaStream_t stream, int counter_slot) {
-    using CFG = SweepConfig<MODE, DPAD, TN, NG, CW>;
+    using CFG = SweepConfig<MODE, DPAD, TN, NG, CW, ALIAS>;
     using MT = ModeTraits<MODE>;
+    constexpr TileType kType = BF16 ? TileType::kBF16 : TileType::kF16;
     auto build = [&](int t, int box_rows) -> int {
         const TensorArg& a = tensors[t];
         if (!a.ptr) return 0;
         int rc = check_strides(a.strides, a.ptr);
         if (rc) return rc;
-        return make_tile_map(&prm.map[t], a.ptr, BF16, g->D, a.q_side ? g->Nq : g->Nk,
+        return make_tile_map(&prm.map[t], a.ptr, kType, g->D, a.q_side ? g->Nq : g->Nk,
                              a.q_side ? g->Hq : g->Hkv, g->B, a.strides[2], a.strides[1],
                              a.strides[0], box_rows);
     };
@@ -147,72 +123,64 @@ static int launch_sweep(const bob_sm100_geom* g, SweepParams& prm, const TensorA
         int rc = build(own_tensor<MODE>(i), 128);
         if (rc) return rc;
     }
+    if (CFG::OWN_OUT) {
+        int rc = build(kTOUT, 128);
+        if (rc) return rc;
+    }
     for (int i = 0; i < MT::NOTH; ++i) {
         int rc = build(other_tensor<MODE>(i), TN);
         if (rc) return rc;
     }
+    // results: contiguous [B, H, N, D]
+    const int n_own = MT::COL ? g->Nk : g->Nq, heads = MT::COL ? g->Hkv : g->Hq;
+    auto result = [&](int i, const void* ptr, TileType type) -> int {
+        const int64_t sn = g->D, sh = sn * n_own;
+        return make_tile_map(&prm.res_map[i], ptr, type, g->D, n_own, heads, g->B, sn, sh, sh * heads, 128);
+    };
+    if (CFG::N_STAGED > 0) { if (int rc = result(0, prm.res0, kType)) return rc; }
+    if (CFG::N_STAGED > 1) { if (int rc = result(1, prm.res1, kType)) return rc; }
+    if (CFG::STAGED_PK && prm.pk) { if (int rc = result(2, prm.pk, TileType::kF32)) return rc; }
+    if (g->device < 0 || g->device >= 64) return kErrDevice;
     // The second backward has a build of its own for the usual case of three defined tangents.
     constexpr bool kSecond = (MODE == kBwd2Row || MODE == kBwd2Col);
     const bool allt = kSecond && prm.has_uq && prm.has_uk && prm.has_uv;
-    auto kernel = allt ? sweep_kernel<MODE, DPAD, TN, BF16, NG, CW, kSecond>
-                       : sweep_kernel<MODE, DPAD, TN, BF16, NG, CW, false>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM_BYTES) !=
-        cudaSuccess)
-        return kErrAttr;
-    if constexpr (CFG::REBALANCE) {
-        // The kernel's warpgroups trade registers after launch; the trade only balances (and the
-        // pointwise warps' request can only ever be met) if the kernel was built with the register
-        // count the trade assumes.  Refuse to launch otherwise.
-        cudaFuncAttributes a;
-        const int regs_at_launch = cudaFuncGetAttributes(&a, kernel) == cudaSuccess ? a.numRegs : 0;
-        if (regs_at_launch * CFG::NTHREADS < 256 * CFG::REGS_POINTWISE + 128 * CFG::REGS_ROLE) return kErrRegs;
-    }
-    // CTAs take work items in rounds (see the kernel): gridDim.x items per round.
-    const int n_own = MT::COL ? g->Nk : g->Nq;
-    const long long items = (long long)((n_own + 127) / 128) * (MT::COL ? g->Hkv : g->Hq) * g->B;
+    auto kernel = allt ? sweep_kernel<MODE, DPAD, TN, BF16, NG, CW, ALIAS, kSecond>
+                       : sweep_kernel<MODE, DPAD, TN, BF16, NG, CW, ALIAS, false>;
+    static std::atomic<uint64_t> done[2];
+    if (int rc = prepare_kernel<CFG>(kernel, g->device, done[allt])) return rc;
+    const long long items = (long long)((n_own + 127) / 128) * heads * g->B;
     if (items > 0x7fffffffLL) return kErrGeom;
     const int sms = sm_count(g->device);
     if (sms <= 0) return kErrDevice;
-    // One persistent CTA per SM whenever there are more items than SMs.  (With the earlier static
-    // assignment of items to CTAs, head dim 128 was ~4 % faster with one CTA per item and the hardware's
-    // own placement; fed from the counter the persistent launch is 0.3-2 % faster there too.)
+    // One persistent CTA per SM whenever there are more items than SMs; it takes items, longest first, from a
+    // counter in the status block (zeroed with it).
     const bool persistent = items > sms;
     dim3 grid((unsigned)(persistent ? sms : items), 1, 1);
-    // Persistent CTAs take items, longest first, from a counter in the status block (zeroed with it);
-    // column-owned ones with a parking area instead split the item list evenly (see the kernel).
     prm.work_counter = persistent ? prm.status + kCounterWord0 + counter_slot : nullptr;
-    prm.sk_span = 0;
-    if (MT::COL && persistent && prm.sk_park && prm.sk_flags) {
-        prm.sk_span = even_split_span(g, prm.delta_off, TN, (int)grid.x);
-        if (prm.sk_span > 0 &&
-            cudaMemsetAsync(prm.sk_flags, 0, even_split_flag_bytes(g), stream) != cudaSuccess)
-            return kErrLaunch;
-    }
     kernel<<<grid, CFG::NTHREADS, CFG::SMEM_BYTES, stream>>>(prm);
     return cudaGetLastError() == cudaSuccess ? 0 : kErrLaunch;
 }
 
 // Tile table (template arguments: head dim, swept-tile width, dtype, pointwise groups, score columns
-// per pointwise thread).
+// per pointwise thread, operands over the scores).
 // Head dim <= 64.  Forward: 128-wide tiles, two groups of 128 threads, each thread a whole row, each
-// group its own online softmax and output accumulator.  First backward: 128-wide tiles, one group of
-// 512 threads (more warps per scheduler measured better than fewer threads holding more columns).
-// Second backward: four score accumulators, four operands and two outputs fill tensor memory at
+// group its own online softmax and output accumulator.  First backward: 64-wide tiles, two groups of 256
+// threads.  Second backward: four score accumulators, four operands and two outputs fill tensor memory at
 // 64-wide tiles; one group of 256 threads holds a whole tile's columns at 208 registers.
-// Head dim 128.  Forward: 64-wide tiles, two groups, a row per thread.  First backward: 64-wide tiles.
-// Second backward: tensor memory (512 columns) leaves room for 32-wide tiles only.
+// Head dim 128.  Forward and first backward as above, with the operands over the scores: the output
+// accumulators take half of tensor memory.  Second backward: room for 32-wide tiles only.
 template <int MODE, bool BF16>
 static int dispatch(const bob_sm100_geom* g, SweepParams& prm, const TensorArg* tensors,
                     cudaStream_t stream, int counter_slot) {
     constexpr bool kSecond = (MODE == kBwd2Row || MODE == kBwd2Col);
     if (g->D <= 64) {
-        if constexpr (kSecond)           return launch_sweep<MODE, 64, 64, BF16, 1, 32>(g, prm, tensors, stream, counter_slot);
-        else if constexpr (MODE == kFwd) return launch_sweep<MODE, 64, 128, BF16, 2, 128>(g, prm, tensors, stream, counter_slot);
-        else                             return launch_sweep<MODE, 64, 128, BF16, 1, 32>(g, prm, tensors, stream, counter_slot);
+        if constexpr (kSecond)           return launch_sweep<MODE, 64, 64, BF16, 1, 32, false>(g, prm, tensors, stream, counter_slot);
+        else if constexpr (MODE == kFwd) return launch_sweep<MODE, 64, 128, BF16, 2, 128, false>(g, prm, tensors, stream, counter_slot);
+        else                             return launch_sweep<MODE, 64, 64, BF16, 2, 32, false>(g, prm, tensors, stream, counter_slot);
     }
-    if constexpr (kSecond)           return launch_sweep<MODE, 128, 32, BF16>(g, prm, tensors, stream, counter_slot);
-    else if constexpr (MODE == kFwd) return launch_sweep<MODE, 128, 64, BF16, 2, 64>(g, prm, tensors, stream, counter_slot);
-    else                             return launch_sweep<MODE, 128, 64, BF16>(g, prm, tensors, stream, counter_slot);
+    if constexpr (kSecond)           return launch_sweep<MODE, 128, 32, BF16, 1, 16, false>(g, prm, tensors, stream, counter_slot);
+    else if constexpr (MODE == kFwd) return launch_sweep<MODE, 128, 128, BF16, 2, 128, true>(g, prm, tensors, stream, counter_slot);
+    else                             return launch_sweep<MODE, 128, 64, BF16, 2, 32, true>(g, prm, tensors, stream, counter_slot);
 }
 
 template <int MODE>
@@ -222,11 +190,10 @@ static int dispatch_dtype(const bob_sm100_geom* g, SweepParams& prm, const Tenso
                                       : dispatch<MODE, false>(g, prm, tensors, stream, counter_slot);
 }
 
-// Only builds with -DBOB_PHASE_TIMERS or -DBOB_TRACE (never the shipped library) read a device pointer (hex) from
-// BOB_SM100_PHASE_PTR: 24 cycle counters (12 of a pointwise thread, then 12 of the MMA warp).
-static long long* phase_pointer() {
-#if defined(BOB_PHASE_TIMERS) || defined(BOB_TRACE)
-    const char* e = std::getenv("BOB_SM100_PHASE_PTR");
+// Only builds with -DBOB_TRACE (never the shipped library) read a device pointer (hex) from BOB_SM100_TRACE_PTR.
+static long long* trace_pointer() {
+#if defined(BOB_TRACE)
+    const char* e = std::getenv("BOB_SM100_TRACE_PTR");
     return e ? reinterpret_cast<long long*>(std::strtoull(e, nullptr, 16)) : nullptr;
 #else
     return nullptr;
@@ -266,14 +233,16 @@ static void fill_common(const bob_sm100_geom* g, SweepParams& p, void* workspace
     p.B = g->B; p.Hq = g->Hq; p.Hkv = g->Hkv; p.G = g->Hq / g->Hkv; p.Nq = g->Nq; p.Nk = g->Nk;
     p.D = g->D;
     p.is_causal = g->is_causal ? 1 : 0;
-    p.window = g->window;
-    // Beyond +-2^30 every pair is masked the same way as at the bound (sequence lengths are far
-    // smaller), and 32-bit position arithmetic in the kernels cannot overflow.
-    const int64_t d = g->q_offset - g->k_offset;
-    p.delta_off = static_cast<int>(d > (1 << 30) ? (1 << 30) : (d < -(1 << 30) ? -(1 << 30) : d));
+    // Lengths are at most 2^28.  Beyond +-2^29 the causal condition has the same outcome for every pair as at
+    // the bound; a window moves with the part of the offset that is cut off, and one beyond 2^30 excludes
+    // nothing.  32-bit position arithmetic in the kernels then cannot overflow.
+    const int64_t kBound = 1 << 29, d = g->q_offset - g->k_offset;
+    const int64_t dc = std::min(kBound, std::max(-kBound, d));
+    p.delta_off = static_cast<int>(dc);
+    p.window = g->window > 0 ? static_cast<int>(std::min<int64_t>(1 << 30, std::max<int64_t>(1, g->window - (d - dc)))) : 0;
     p.scale = g->scale;
     p.status = static_cast<int*>(workspace);
-    p.phase_cycles = phase_pointer();
+    p.trace = trace_pointer();
 }
 
 static void set_strided(const void*& dst, long long& sb, long long& sh, long long& sn,
@@ -309,27 +278,16 @@ extern "C" const char* bob_sm100_error_string(int code) {
         case 77: return "device: the self-test's wait ran out (as it is meant to)";
         case kStatusTimeoutLoad: return "device: a wait for a TMA load ran out";
         case kStatusTimeoutMma: return "device: a wait in the MMA issuer ran out";
+        case kStatusMisaligned: return "device: shared memory is not 1024-byte aligned";
         case kStatusTimeoutPw: return "device: a wait in the pointwise threads ran out";
         default: return code < -1000 ? "cuTensorMapEncodeTiled failed" : "unknown code";
     }
 }
 
-// Bytes of the even-split area (flags, then parked partials) a stage's column-owned kernel may use.
-static size_t even_split_bytes(const bob_sm100_geom* g) {
-#ifndef BOB_EVEN_SPLIT
-    (void)g;
-    return 0;
-#endif
-    const int sms = sm_count(g->device);
-    if (sms <= 0 || !col_launch_is_persistent(g, sms)) return 0;
-    return even_split_flag_bytes(g) + even_split_park_bytes(sms);
-}
-
 extern "C" size_t bob_sm100_workspace_bytes(int stage, const bob_sm100_geom* g) {
     if (!g || g->B <= 0 || g->Hq <= 0 || g->Hkv <= 0 || g->Nq <= 0 || g->Nk <= 0) return 0;
     size_t bytes = kStatusBlock;
-    if (stage == BOB_SM100_STAGE_BWD2) bytes = bwd2_workspace_bytes_unsplit(g);
-    if (stage == BOB_SM100_STAGE_BWD1 || stage == BOB_SM100_STAGE_BWD2) bytes += even_split_bytes(g);
+    if (stage == BOB_SM100_STAGE_BWD2) bytes = bwd2_workspace_bytes(g);
     return bytes;
 }
 
@@ -406,6 +364,7 @@ extern "C" int bob_sm100_bwd1(const bob_sm100_geom* g, const void* q, const void
     t[kTK] = {k, g->k_strides, false};
     t[kTV] = {v, g->v_strides, false};
     t[kTDO] = {dO, g->do_strides, true};
+    t[kTOUT] = {out, g->out_strides, true};
 
     SweepParams p;
     fill_common(g, p, workspace);
@@ -413,24 +372,18 @@ extern "C" int bob_sm100_bwd1(const bob_sm100_geom* g, const void* q, const void
     p.lse = const_cast<float*>(lse);
     p.delta = delta;
     p.pk = pk;
-    set_strided(p.out, p.out_sb, p.out_sh, p.out_sn, out, g->out_strides);
-    set_strided(p.dO, p.dO_sb, p.dO_sh, p.dO_sn, dO, g->do_strides);
     p.res0 = dQ;
     rc = dispatch_dtype<kBwd1Row>(g, p, t, s, 0);   // dQ and delta
     if (rc) return rc;
     p.res0 = dK;
     p.res1 = dV;
-    if (even_split_bytes(g)) {
-        p.sk_flags = reinterpret_cast<int*>(static_cast<char*>(workspace) + kStatusBlock);
-        p.sk_park = reinterpret_cast<float*>(static_cast<char*>(workspace) + kStatusBlock + even_split_flag_bytes(g));
-    }
     return dispatch_dtype<kBwd1Col>(g, p, t, s, 1); // dK and dV (reads delta)
 }
 
 int bob::bwd2_impl(const bob_sm100_geom* g, const void* q, const void* k, const void* v, const void* out,
                    const float* lse, const float* delta, const float* pk, const void* dO, const void* dQ,
                    const void* uQ, const void* uK, const void* uV, void* Qbar, void* Kbar, void* Vbar,
-                   void* dObar, void* workspace, void* stream, int* sticky, int part, bool allow_split) {
+                   void* dObar, void* workspace, void* stream, int* sticky, int part) {
     int rc = check_geom(g);
     if (rc) return rc;
     if (!q || !k || !v || !out || !lse || !delta || !pk || !dO || !dQ || !Qbar || !Kbar || !Vbar || !dObar)
@@ -476,17 +429,12 @@ int bob::bwd2_impl(const bob_sm100_geom* g, const void* q, const void* k, const 
     if (part & kPartCol) {
         p.res0 = Kbar;
         p.res1 = Vbar;
-        if (allow_split && even_split_bytes(g)) {
-            char* area = static_cast<char*>(workspace) + bwd2_workspace_bytes_unsplit(g);
-            p.sk_flags = reinterpret_cast<int*>(area);
-            p.sk_park = reinterpret_cast<float*>(area + even_split_flag_bytes(g));
-        }
         rc = dispatch_dtype<kBwd2Col>(g, p, t, s, 1);   // Kbar, Vbar (reads alpha, ecirc)
     }
     return rc;
 }
 
-size_t bob::bwd2_workspace_bytes_unsplit(const bob_sm100_geom* g) {
+size_t bob::bwd2_workspace_bytes(const bob_sm100_geom* g) {
     return kStatusBlock + 2 * round256(static_cast<size_t>(g->B) * g->Hq * g->Nq * sizeof(float));
 }
 
@@ -496,7 +444,7 @@ extern "C" int bob_sm100_bwd2(const bob_sm100_geom* g, const void* q, const void
                               void* Qbar, void* Kbar, void* Vbar, void* dObar, void* workspace,
                               void* stream) {
     return bwd2_impl(g, q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV, Qbar, Kbar, Vbar, dObar, workspace,
-                     stream, g ? sticky_word(g->device, true) : nullptr, kPartBoth, true);
+                     stream, g ? sticky_word(g->device, true) : nullptr, kPartBoth);
 }
 
 extern "C" int bob_sm100_bwd2_part(int part, const bob_sm100_geom* g, const void* q, const void* k,
@@ -505,5 +453,5 @@ extern "C" int bob_sm100_bwd2_part(int part, const bob_sm100_geom* g, const void
                                    const void* uK, const void* uV, void* Qbar, void* Kbar, void* Vbar,
                                    void* dObar, void* workspace, void* stream) {
     return bwd2_impl(g, q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV, Qbar, Kbar, Vbar, dObar, workspace,
-                     stream, g ? sticky_word(g->device, true) : nullptr, part, true);
+                     stream, g ? sticky_word(g->device, true) : nullptr, part);
 }

@@ -65,14 +65,13 @@ extern "C" int bob_sm100_bwd2_noalloc(const bob_sm100_geom* g, const void* q, co
     if (g->B <= 0 || g->Hq <= 0 || g->Nq <= 0) return -2;
     const size_t rows = static_cast<size_t>(g->B) * static_cast<size_t>(g->Hq) * static_cast<size_t>(g->Nq);
     if (rows > kMaxRows) return -12;                               // larger than the built-in scratch
-    if (bob::bwd2_workspace_bytes_unsplit(g) > kNoAllocScratchBytes) return -12;
+    if (bob::bwd2_workspace_bytes(g) > kNoAllocScratchBytes) return -12;
     void* scratch = nullptr;
     const int rc = scratch_address(g->device, &scratch);
     if (rc) return rc;
-    // no host-visible status word (its set-up page-locks memory) and no division of long work items
-    // (that needs a larger workspace): this path touches nothing but the fixed array
+    // no host-visible status word (its set-up page-locks memory): this path touches nothing but the fixed array
     return bob::bwd2_impl(g, q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV, Qbar, Kbar, Vbar, dObar,
-                          scratch, stream, nullptr, bob::kPartBoth, false);
+                          scratch, stream, nullptr, bob::kPartBoth);
 }
 
 // Waits for `stream`, then returns the status word the last bob_sm100_bwd2_noalloc call on `device`

@@ -128,6 +128,16 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
           "r"(batch), "r"(bar)
         : "memory");
 }
+// 4-D tiled store, this CTA's shared memory -> global; rows and columns outside the tensor are clipped.
+// The shared memory may be reused after bulk_commit() and bulk_wait_read() by the same thread.
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int x, int row, int head, int batch) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+        ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(row), "r"(head), "r"(batch), "r"(src)
+        : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }

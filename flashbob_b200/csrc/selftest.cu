@@ -200,9 +200,9 @@ extern "C" int bob_sm100_selftest(const void* a, const void* b, int is_bf16, flo
     using namespace bob;
     if (!a || !b || !out || !status) return -1;
     SelftestMaps maps;
-    int rc = make_tile_map(&maps.a, a, is_bf16 != 0, 64, 128, 1, 1, 64, 64 * 128, 64 * 128, 128);
+    int rc = make_tile_map(&maps.a, a, is_bf16 ? TileType::kBF16 : TileType::kF16, 64, 128, 1, 1, 64, 64 * 128, 64 * 128, 128);
     if (rc) return rc;
-    rc = make_tile_map(&maps.b, b, is_bf16 != 0, 64, 64, 1, 1, 64, 64 * 64, 64 * 64, 64);
+    rc = make_tile_map(&maps.b, b, is_bf16 ? TileType::kBF16 : TileType::kF16, 64, 64, 1, 1, 64, 64 * 64, 64 * 64, 64);
     if (rc) return rc;
     const int smem = 16384 + 2 * 8192 + 16384 + 64 + 1024;
     auto kernel = selftest_kernel;

@@ -31,10 +31,11 @@ inline EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Tile box = 64 head-dim elements (one 128-byte swizzle span) x box_rows rows of one head.
-// Elements outside the tensor (rows past N, head-dim elements past D) read as zero.
-// Returns 0 on success.
-inline int make_tile_map(CUtensorMap* map, const void* base, bool is_bf16, int64_t D, int64_t N,
+// Tile box = one 128-byte swizzle span of head-dim elements (64 of 16 bits, 32 of fp32) x box_rows rows of
+// one head.  Elements outside the tensor (rows past N, head-dim elements past D) read as zero and are
+// not written.  Returns 0 on success.
+enum class TileType { kF16, kBF16, kF32 };
+inline int make_tile_map(CUtensorMap* map, const void* base, TileType type, int64_t D, int64_t N,
                          int64_t H, int64_t B, int64_t stride_n, int64_t stride_h,
                          int64_t stride_b, int box_rows) {
     EncodeTiledFn fn = encode_tiled_fn();
@@ -44,14 +45,16 @@ inline int make_tile_map(CUtensorMap* map, const void* base, bool is_bf16, int64
     if (H == 1) stride_h = stride_n * N;
     if (B == 1) stride_b = stride_h * H;
     if (N == 1) stride_n = D < 8 ? 8 : D;
-    if ((stride_n * 2) % 16 || (stride_h * 2) % 16 || (stride_b * 2) % 16) return -102;
+    const int esize = type == TileType::kF32 ? 4 : 2;
+    if ((stride_n * esize) % 16 || (stride_h * esize) % 16 || (stride_b * esize) % 16) return -102;
     if (stride_n <= 0 || stride_h <= 0 || stride_b <= 0) return -102;
     cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)N, (cuuint64_t)H, (cuuint64_t)B};
-    cuuint64_t strides[3] = {(cuuint64_t)stride_n * 2, (cuuint64_t)stride_h * 2,
-                             (cuuint64_t)stride_b * 2};
-    cuuint32_t box[4] = {64u, (cuuint32_t)box_rows, 1u, 1u};
+    cuuint64_t strides[3] = {(cuuint64_t)(stride_n * esize), (cuuint64_t)(stride_h * esize),
+                             (cuuint64_t)(stride_b * esize)};
+    cuuint32_t box[4] = {128u / esize, (cuuint32_t)box_rows, 1u, 1u};
     cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
-    CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+    CUresult r = fn(map, type == TileType::kF32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                       : type == TileType::kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                     4, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
