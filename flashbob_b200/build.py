@@ -19,7 +19,7 @@ CSRC = PKG / "csrc"
 LIB = PKG / "libbob_sm100.so"
 TORCH_MODULE = PKG / "bob_torch.so"
 SOURCES = ("api.cu", "selftest.cu", "noalloc.cu")
-HEADERS = ("ptx.cuh", "sweep.cuh", "tmap.h", "internal.h")
+HEADERS = ("ptx.cuh", "sweep.cuh", "decode.cuh", "tmap.h", "internal.h")
 
 
 def _nvcc() -> str:

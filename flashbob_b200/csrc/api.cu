@@ -1,5 +1,6 @@
 // Host side of the C ABI: argument checks, tensor-map construction and kernel dispatch.
 #include "internal.h"
+#include "decode.cuh"
 #include "sweep.cuh"
 #include "tmap.h"
 
@@ -228,10 +229,7 @@ int* sticky_word(int device, bool create) {
     return create ? dev[device] : host[device];
 }
 
-static void fill_common(const bob_sm100_geom* g, SweepParams& p, void* workspace) {
-    std::memset(&p, 0, sizeof(p));
-    p.B = g->B; p.Hq = g->Hq; p.Hkv = g->Hkv; p.G = g->Hq / g->Hkv; p.Nq = g->Nq; p.Nk = g->Nk;
-    p.D = g->D;
+static void fill_mask(const bob_sm100_geom* g, SweepParams& p) {
     p.is_causal = g->is_causal ? 1 : 0;
     // Lengths are at most 2^28.  Beyond +-2^29 the causal condition has the same outcome for every pair as at
     // the bound; a window moves with the part of the offset that is cut off, and one beyond 2^30 excludes
@@ -240,6 +238,13 @@ static void fill_common(const bob_sm100_geom* g, SweepParams& p, void* workspace
     const int64_t dc = std::min(kBound, std::max(-kBound, d));
     p.delta_off = static_cast<int>(dc);
     p.window = g->window > 0 ? static_cast<int>(std::min<int64_t>(1 << 30, std::max<int64_t>(1, g->window - (d - dc)))) : 0;
+}
+
+static void fill_common(const bob_sm100_geom* g, SweepParams& p, void* workspace) {
+    std::memset(&p, 0, sizeof(p));
+    p.B = g->B; p.Hq = g->Hq; p.Hkv = g->Hkv; p.G = g->Hq / g->Hkv; p.Nq = g->Nq; p.Nk = g->Nk;
+    p.D = g->D;
+    fill_mask(g, p);
     p.scale = g->scale;
     p.status = static_cast<int*>(workspace);
     p.trace = trace_pointer();
@@ -248,6 +253,92 @@ static void fill_common(const bob_sm100_geom* g, SweepParams& p, void* workspace
 static void set_strided(const void*& dst, long long& sb, long long& sh, long long& sn,
                         const void* ptr, const int64_t* s) {
     dst = ptr; sb = s[0]; sh = s[1]; sn = s[2];
+}
+
+// ---- forward with a few query rows ------------------------------------------------------------------
+// Up to kDecodeRows query rows per head go to decode_kernel whatever the number of keys: the sweep kernel would
+// do the work of 128 rows for them.  A head's keys are divided until kDecodeCtas CTAs are there (two are resident
+// per SM), but not below one round of a CTA's warps.
+constexpr int kDecodeCtas = 4 * 148;
+struct DecodePlan { int k_lo, k_hi, splits, split_keys; size_t acc_offset, bytes; };     // offsets in the workspace
+
+static DecodePlan decode_plan(const bob_sm100_geom* g) {
+    DecodePlan d = {};
+    SweepParams p;
+    fill_mask(g, p);
+    int64_t lo = 0, hi = g->Nk;                  // keys that any of the rows attends to
+    if (p.is_causal) {
+        hi = std::min<int64_t>(hi, (int64_t)g->Nq + p.delta_off);
+        if (p.window > 0) lo = std::max<int64_t>(0, (int64_t)p.delta_off - p.window + 1);
+    }
+    if (hi < lo) hi = lo = 0;
+    d.k_lo = (int)lo; d.k_hi = (int)hi;
+    const int dpad = g->D <= 32 ? 32 : (g->D <= 64 ? 64 : 128);
+    const int64_t round = decode_round(dpad, g->Nq), rounds = std::max<int64_t>(1, (hi - lo + round - 1) / round);
+    const int64_t heads = (int64_t)g->B * g->Hq;
+    const int64_t want = std::min<int64_t>({kDecodeMaxSplits, rounds, std::max<int64_t>(1, kDecodeCtas / heads)});
+    const int64_t per = (rounds + want - 1) / want;
+    d.split_keys = (int)(per * round);
+    d.splits = (int)((rounds + per - 1) / per);
+    d.bytes = kStatusBlock;
+    if (d.splits > 1) {
+        const size_t rows = (size_t)heads * d.splits * g->Nq;
+        const size_t ml_offset = kStatusBlock + round256(heads * sizeof(int));
+        d.acc_offset = ml_offset + round256(rows * 2 * sizeof(float));
+        d.bytes = d.acc_offset + rows * g->D * sizeof(float);
+    }
+    return d;
+}
+
+template <bool BF16>
+static void launch_decode(const bob_sm100_geom* g, const DecodeParams& p, unsigned grid, cudaStream_t s) {
+    auto rows = [&](auto dpad_tag) {
+        constexpr int DPAD = decltype(dpad_tag)::value;
+        if (g->Nq == 1) decode_kernel<DPAD, 1, BF16><<<grid, kDecodeThreads, 0, s>>>(p);
+        else decode_kernel<DPAD, kDecodeRows, BF16><<<grid, kDecodeThreads, 0, s>>>(p);
+    };
+    if (g->D <= 32) rows(IntTag<32>{});
+    else if (g->D <= 64) rows(IntTag<64>{});
+    else rows(IntTag<128>{});
+}
+
+static int run_decode(const bob_sm100_geom* g, const void* q, const void* k, const void* v, void* out, float* lse,
+                      void* workspace, cudaStream_t s) {
+    // the same layouts as the sweep kernels take
+    auto check = [&](const void* ptr, const int64_t* st, int64_t N, int64_t H) -> int {
+        if (int rc = check_strides(st, ptr)) return rc;
+        int64_t sn = st[2], sh = st[1], sb = st[0];
+        return fit_strides(g->D, N, H, g->B, sn, sh, sb, TileType::kF16);
+    };
+    if (int rc = check(q, g->q_strides, g->Nq, g->Hq)) return rc;
+    if (int rc = check(k, g->k_strides, g->Nk, g->Hkv)) return rc;
+    if (int rc = check(v, g->v_strides, g->Nk, g->Hkv)) return rc;
+    const DecodePlan d = decode_plan(g);
+    const int64_t heads = (int64_t)g->B * g->Hq, grid = heads * d.splits;
+    if (grid > 0x7fffffffLL) return kErrGeom;
+    SweepParams m;
+    fill_mask(g, m);
+    char* ws = static_cast<char*>(workspace);
+    DecodeParams p = {};
+    p.q = static_cast<const uint16_t*>(q); p.q_sb = g->q_strides[0]; p.q_sh = g->q_strides[1]; p.q_sn = g->q_strides[2];
+    p.k = static_cast<const uint16_t*>(k); p.k_sb = g->k_strides[0]; p.k_sh = g->k_strides[1]; p.k_sn = g->k_strides[2];
+    p.v = static_cast<const uint16_t*>(v); p.v_sb = g->v_strides[0]; p.v_sh = g->v_strides[1]; p.v_sn = g->v_strides[2];
+    p.Hq = g->Hq; p.G = g->Hq / g->Hkv; p.Nq = g->Nq; p.D = g->D;
+    p.causal = m.is_causal; p.window = m.window; p.delta_off = m.delta_off;
+    p.k_lo = d.k_lo; p.k_hi = d.k_hi; p.splits = d.splits; p.split_keys = d.split_keys;
+    p.scale = g->scale;
+    p.out = static_cast<uint16_t*>(out);
+    p.lse = lse;
+    p.status = reinterpret_cast<int*>(ws);
+    if (d.splits > 1) {
+        p.arrived = reinterpret_cast<int*>(ws + kStatusBlock);
+        p.part_ml = reinterpret_cast<float*>(ws + kStatusBlock + round256(heads * sizeof(int)));
+        p.part_acc = reinterpret_cast<float*>(ws + d.acc_offset);
+        if (cudaMemsetAsync(p.arrived, 0, heads * sizeof(int), s) != cudaSuccess) return kErrLaunch;
+    }
+    if (g->dtype == BOB_SM100_BF16) launch_decode<true>(g, p, (unsigned)grid, s);
+    else launch_decode<false>(g, p, (unsigned)grid, s);
+    return cudaGetLastError() == cudaSuccess ? 0 : kErrLaunch;
 }
 
 }  // namespace bob
@@ -288,6 +379,7 @@ extern "C" size_t bob_sm100_workspace_bytes(int stage, const bob_sm100_geom* g) 
     if (!g || g->B <= 0 || g->Hq <= 0 || g->Hkv <= 0 || g->Nq <= 0 || g->Nk <= 0) return 0;
     size_t bytes = kStatusBlock;
     if (stage == BOB_SM100_STAGE_BWD2) bytes = bwd2_workspace_bytes(g);
+    if (stage == BOB_SM100_STAGE_FWD && g->Nq <= kDecodeRows) bytes = decode_plan(g).bytes;
     return bytes;
 }
 
@@ -329,11 +421,13 @@ extern "C" int bob_sm100_fwd(const bob_sm100_geom* g, const void* q, const void*
     DeviceGuard guard(g->device);
     if (!guard.ok) return kErrDevice;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int* sticky = sticky_word(g->device, true);
+    if (g->Nq <= kDecodeRows) return run_decode(g, q, k, v, out, lse, workspace, s);
     if ((rc = begin_call(workspace, s))) return rc;
 
     SweepParams p;
     fill_common(g, p, workspace);
-    p.sticky = sticky_word(g->device, true);
+    p.sticky = sticky;
     p.lse = lse;
     p.res0 = out;
     TensorArg t[kNumTensors] = {};
