@@ -189,6 +189,7 @@ struct SweepConfig {
     static constexpr int SLOT_ROOM = (SMEM_LIMIT - OWN_TILES * OWN_TILE_BYTES - IO_BYTES - RED_FLOATS * 4 - MISC_BYTES) / (SLOT_BYTES + NSTAT * TN * 4);
     static constexpr int NSLOT = SLOT_ROOM >= MAX_SLOTS ? MAX_SLOTS : SLOT_ROOM;
     static_assert(SPLIT_KV ? NSLOT >= 2 * NG : NSLOT > NG, "score products run up to NG tiles ahead");
+    static_assert(NG * SLOTS_PER_TILE <= NSLOT, "a group's step through the ring wraps at most once");
     static constexpr int OFF_OWN = 0;
     static constexpr int OFF_OTH = OFF_OWN + OWN_TILES * OWN_TILE_BYTES;
     static constexpr int OFF_IO = OFF_OTH + NSLOT * SLOT_BYTES;                 // staged results / epilogue operands
@@ -252,7 +253,6 @@ __device__ __forceinline__ void store16_from_float(void* base, long long elem_of
     p[0] = a; p[1] = b;
 }
 
-template <bool V> struct BoolTag { static constexpr bool value = V; };
 template <int V> struct IntTag { static constexpr int value = V; };
 
 template <int MODE, int DPAD, int TN, bool BF16, int NG, int CW, bool ALIAS, bool ALLT = false>
@@ -372,6 +372,10 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
     auto has_tensor = [&](int t) {
         return t == kTUQ ? has_uq : (t == kTUK ? has_uk : (t == kTUV ? has_uv : true));
     };
+
+    // -lse in log2 units.  A row without keys has lse = -inf: kept finite, so that its scores, all masked to -inf, still
+    // give probability zero.
+    auto neg_log2 = [](float lse) { return lse == -INFINITY ? 3.0e38f : -lse * kLog2e; };
 
     // ---- set-up ------------------------------------------------------------------------------
     if (tid == 0) {
@@ -564,7 +568,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                         for (int k = 0; k < RPL; ++k) {
                             const int r = lane + 32 * k;
                             if (r < TN) {
-                                sb[r] = -(st_l2[k] * kLog2e); sb[TN + r] = -st_d[k];
+                                sb[r] = neg_log2(st_l2[k]); sb[TN + r] = -st_d[k];
                                 if constexpr (BWD2) { sb[2 * TN + r] = -st_al[k]; sb[3 * TN + r] = -st_ec[k]; }
                             }
                         }
@@ -866,7 +870,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             wait(bar_pw_all, pw_all_phase, kStatusTimeoutPw);
             pw_all_phase ^= 1u;
         };
-        int s = 0, par = 0;                      // slot of the next tile, parity of its use
+        int s = 0, par = 0;                      // slot of the item's next tile, parity of its use
         int last_s = -1, last_par = 0;           // !ALIAS: my group's last tile, whose products must have read its operands
         uint32_t sc_par = 0;                     // parity of my group's next scores
         int n_live = 0;                          // items with at least one tile finished so far
@@ -926,10 +930,10 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             }
             if (grp == 0 && sp == 0 && own_ok) p.delta[row_stat] = dlt;
             ndlt = -dlt;
-            nL2 = -l_row * kLog2e;
+            nL2 = neg_log2(l_row);
         }
         if constexpr (MODE == kBwd2Row) {
-            if (own_ok) { nL2 = -p.lse[row_stat] * kLog2e; ndlt = -p.delta[row_stat]; }
+            if (own_ok) { nL2 = neg_log2(p.lse[row_stat]); ndlt = -p.delta[row_stat]; }
         }
         // Own tile 0 into tensor memory (see SweepConfig::OWN_TM): once the item's own tiles have landed,
         // every thread copies its share of its own row, 16 elements (two 16-byte chunks of the swizzled
@@ -968,9 +972,12 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
         const long long tile_row0 = ((long long)batch * p.Hq + head) * p.Nq + own0;   // first row of the contiguous results
         (void)io_out; (void)io_dq; (void)tile_row0;
 
-        // One swept tile.  FULL: every (row, column) of the tile pair is unmasked and in range.
-        auto tile_body = [&](auto full_tag, int it, int tile) {
-            constexpr bool FULL = decltype(full_tag)::value;
+        // One swept tile.  full: every (row, column) of the tile pair is unmasked and in range.  Elsewhere masked
+        // scores become -inf, which makes their probabilities zero.  One body serves both: a second, unrolled copy
+        // for masked tiles cost more in instruction fetches than it saved in selects (a masked tile of the forward took
+        // 4800 cycles longer than a full one, and every causal item has one; with one body B=8 H=12 S=1024 D=64 training
+        // went from 151.7 to 134.3 us, S=8192 with a window of 1024 from 274.3 to 254.8 us).
+        auto tile_body = [&](const bool full, int it, int tile, int s, int par) {
             const int oth0 = tile * TN;
 
             BOB_TR(0)
@@ -982,13 +989,9 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             // ---- which of my columns are unmasked --------------------------------------------
             // dist = query position - key position; unmasked iff in range and, when causal,
             // 0 <= dist (< window)
-            // Up to 64 columns per thread: a bit mask; more (forward, 128): the range itself.
-            using mask_t = typename std::conditional<(CW > 32), unsigned long long, uint32_t>::type;
-            constexpr mask_t kAllCols = ~mask_t(0) >> (CW >= 64 ? 0 : 8 * (int)sizeof(mask_t) - CW);
-            mask_t vmask = kAllCols;
-            int mlo = 0, mhi = CW - 1;
-            if constexpr (!FULL) {
-                mhi = min(CW - 1, n_oth - (oth0 + col0) - 1);
+            uint32_t vmask[(CW + 31) / 32];          // bit c % 32 of word c / 32: column c of mine is unmasked
+            if (!full) {
+                int mlo = 0, mhi = min(CW - 1, n_oth - (oth0 + col0) - 1);
                 if (causal) {
                     if constexpr (!COL) {
                         const int d0 = own_idx + doff - (oth0 + col0);       // dist falls with the column
@@ -1000,16 +1003,18 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                         if (window > 0) mhi = min(mhi, window - 1 - d0);
                     }
                 }
-                if (!own_ok) { mlo = 1; mhi = 0; }
-                if constexpr (CW <= 64)
-                    vmask = (mhi >= mlo) ? ((kAllCols >> (CW - 1 - mhi)) & (kAllCols << mlo)) : mask_t(0);
+                if (!own_ok) mhi = -1;
+                #pragma unroll
+                for (int k = 0; k < (CW + 31) / 32; ++k) {
+                    const int lo = max(mlo - 32 * k, 0), hi = min(mhi - 32 * k, 31);
+                    vmask[k] = hi >= lo ? (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo) : 0u;
+                }
             }
-            auto valid = [&](int c) -> bool {        // column c of mine is unmasked (c is a constant after unrolling)
-                if constexpr (FULL) return true;
-                else if constexpr (CW <= 64) return ((vmask >> c) & 1) != 0;
-                else return c >= mlo && c <= mhi;
+            // n scores from column c0 of mine on
+            auto mask_scores = [&](float* v, int c0, int n) {
+                #pragma unroll
+                for (int c = 0; c < n; ++c) v[c] = (vmask[(c0 + c) / 32] >> ((c0 + c) % 32)) & 1u ? v[c] : -INFINITY;
             };
-            (void)valid; (void)vmask;
             // The previous products of my group must have read its operands before I write new ones (with ALIAS
             // they have: the scores just read were issued after them).
             auto operands_free = [&]() {
@@ -1028,11 +1033,12 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                     if (lane == 0) mbar_arrive(bar_sc_empty(grp));
                 }
                 BOB_TR(2)
+                if (!full) mask_scores(s_, 0, CW);
                 // largest unmasked score of my row in this tile (the scale is positive)
                 float mr4[4] = {-3.0e38f, -3.0e38f, -3.0e38f, -3.0e38f};     // four chains, for instruction-level parallelism
                 #pragma unroll
                 for (int c = 0; c < CW; c += 2)
-                    mr4[(c >> 1) & 3] = fmaxf(fmaxf(mr4[(c >> 1) & 3], valid(c) ? s_[c] : -3.0e38f), valid(c + 1) ? s_[c + 1] : -3.0e38f);
+                    mr4[(c >> 1) & 3] = fmaxf(fmaxf(mr4[(c >> 1) & 3], s_[c]), s_[c + 1]);
                 const float mr = fmaxf(fmaxf(mr4[0], mr4[1]), fmaxf(mr4[2], mr4[3]));
                 const float mt = fmaxf(mr * c_exp, -1e30f);
                 // move the reference only when the maximum has outgrown it; the whole warp then
@@ -1077,11 +1083,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                     for (int k = 0; k < 8; ++k) {
                         const int c = 16 * h + 2 * k;
                         const float2 x = __ffma2_rn(make_float2(s_[c], s_[c + 1]), cexp2, nm2);
-                        float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                        if constexpr (!FULL) {
-                            pr.x = valid(c) ? pr.x : 0.f;
-                            pr.y = valid(c + 1) ? pr.y : 0.f;
-                        }
+                        const float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
                         sum4[k & 3] = __fadd2_rn(sum4[k & 3], pr);
                         w0[k] = pack2<BF16>(pr.x, pr.y);
                     }
@@ -1144,6 +1146,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                         BOB_TR(2)
                     }
                     float* s_ = in_s[b];
+                    if (!full) mask_scores(s_, RW * half, RW);
                     float* dp_ = in_dp[b];
                     float* f_ = in_f[b];
                     float* cc_ = in_c[b];
@@ -1171,7 +1174,6 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                         #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             const int c = 4 * c4 + 2 * h;          // columns c, c + 1 of this round
-                            const int mc = RW * half + c;          // bit index in vmask
                             const int wi = c >> 1;                 // packed word index inside this round
                             float2 nl2, ndl, nal, nec;
                             (void)nal; (void)nec;
@@ -1187,11 +1189,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                                 ndl = make_float2(ndlt, ndlt);
                             }
                             const float2 x = __ffma2_rn(make_float2(s_[c], s_[c + 1]), cexp2, nl2);
-                            float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                            if constexpr (!FULL) {
-                                pr.x = ((vmask >> mc) & 1u) ? pr.x : 0.f;
-                                pr.y = ((vmask >> (mc + 1)) & 1u) ? pr.y : 0.f;
-                            }
+                            const float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
                             const float2 dps = __fadd2_rn(make_float2(dp_[c], dp_[c + 1]), ndl);
                             if constexpr (MODE == kBwd1Row) {
                                 const float2 ds = __fmul2_rn(pr, dps);
@@ -1265,18 +1263,24 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                 }
                 if (hi > lo) { full_lo = lo; full_hi = hi; }
             }
-            int tile = t_lo;
-            for (int it = 0; it < total; ++it) {
-                if (NG == 1 || (it & 1) == grp) {        // my group's turn
-                    // is the whole 128 x TN tile pair unmasked and inside both tensors?  (uniform per CTA)
-                    const bool full = tile >= full_lo && tile < full_hi;
-                    if (full) tile_body(BoolTag<true>{}, it, tile);
-                    else tile_body(BoolTag<false>{}, it, tile);
+            // my group's tiles; from one to the next, NG tiles and their slots are passed
+            int tile = t_lo + (NG == 2 ? grp : 0), ts = s + (NG == 2 ? grp : 0) * SPT, tp = par;
+            const int n_sweep = t_hi - t_lo;
+            if (ts >= NSLOT) { ts -= NSLOT; tp ^= 1; }
+            if (COL && tile >= t_hi) tile -= n_sweep;
+            for (int it = NG == 2 ? grp : 0; it < total; it += NG) {
+                tile_body(tile >= full_lo && tile < full_hi, it, tile, ts, tp);
+                tile += NG;
+                if (COL && tile >= t_hi) {               // the next head of the group
+                    tile -= n_sweep;
+                    if (NG == 2 && tile >= t_hi) tile -= n_sweep;
                 }
-                if (++tile == t_hi) tile = t_lo;
-                s += SPT;
-                if (s >= NSLOT) { s -= NSLOT; par ^= 1; }
+                ts += NG * SPT;
+                if (ts >= NSLOT) { ts -= NSLOT; tp ^= 1; }
             }
+            const int end = s + total * SPT;
+            par ^= (end / NSLOT) & 1;
+            s = end % NSLOT;
         }
 
         // ---- epilogue ------------------------------------------------------------------------
