@@ -177,6 +177,16 @@ struct SweepConfig {
     static constexpr bool STAGED_PK = MODE == kBwd1Row && DPAD == 64;          // (no room at head dim 128)
     static constexpr int N_STAGED = STAGED_OUT ? (MODE == kBwd1Col || MODE == kBwd2Col ? 2 : 1) : 0;
     static constexpr int IO_BYTES = STAGED_IO ? 32 * 1024 : N_STAGED * OWN_TILE_BYTES + (STAGED_PK ? DPAD * 512 : 0);
+    // Where shared memory has no room for that (head dim 128: both results of the second backward, the epilogue
+    // operands of its row-owned kernel, and pk of the first backward), eight lanes turn their eight rows' 128 bytes
+    // around in registers, so that a warp-wide access touches 4 lines.  With a row per lane it touches 32, and the
+    // row-owned second backward spent 19600 cycles between an item's last tile and the end of its epilogue (a tile
+    // takes 1900), the column-owned one 7100, the first backward 9400; with the rows turned around 13900, 5000 and 6900
+    // (kernels at H=32 S=2048: 184 to 174, 167 to 165 and 88 to 83 us).
+    static constexpr bool TURN_IO = BWD2 && DPAD == 128;
+    static constexpr bool TURN_PK = MODE == kBwd1Row && !STAGED_PK;
+    static_assert(!TURN_IO || DPAD / (NSPLIT * NG) == 64, "128 bytes of a 16-bit row per thread");
+    static_assert(!TURN_PK || DPAD / (NSPLIT * NG) == 32, "128 bytes of an fp32 row per thread");
     // shared memory map (offsets from the 1024-byte aligned base)
     static constexpr int RED_COPIES = MODE == kBwd2Row && DPAD == 64 ? 2 : 1;
     static constexpr int RED_FLOATS = MODE == kFwd ? 8 * 128 : (MODE == kBwd1Row ? NG * NSPLIT * 128 : (MODE == kBwd2Row ? RED_COPIES * 2 * NG * NSPLIT * 128 : 0));
@@ -209,25 +219,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 template <bool BF16>
-__device__ __forceinline__ void load16_as_float(const void* base, long long elem_off, float* v) {
-    const uint4* p = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + elem_off);
-    uint4 a = p[0], b = p[1];
-    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        if constexpr (BF16) {
-            __nv_bfloat162 t = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
-            float2 f = __bfloat1622float2(t);
-            v[2 * i] = f.x; v[2 * i + 1] = f.y;
-        } else {
-            __half2 t = *reinterpret_cast<const __half2*>(&w[i]);
-            float2 f = __half22float2(t);
-            v[2 * i] = f.x; v[2 * i + 1] = f.y;
-        }
-    }
-}
-
-template <bool BF16>
 __device__ __forceinline__ void unpack8_as_float(const uint4 a, float* v) {
     const uint32_t w[4] = {a.x, a.y, a.z, a.w};
     #pragma unroll
@@ -242,15 +233,23 @@ __device__ __forceinline__ void unpack8_as_float(const uint4 a, float* v) {
     }
 }
 
-template <bool BF16>
-__device__ __forceinline__ void store16_from_float(void* base, long long elem_off, const float* v) {
-    uint4 a, b;
-    a.x = pack2<BF16>(v[0], v[1]);   a.y = pack2<BF16>(v[2], v[3]);
-    a.z = pack2<BF16>(v[4], v[5]);   a.w = pack2<BF16>(v[6], v[7]);
-    b.x = pack2<BF16>(v[8], v[9]);   b.y = pack2<BF16>(v[10], v[11]);
-    b.z = pack2<BF16>(v[12], v[13]); b.w = pack2<BF16>(v[14], v[15]);
-    uint4* p = reinterpret_cast<uint4*>(static_cast<uint16_t*>(base) + elem_off);
-    p[0] = a; p[1] = b;
+// Transposes an 8 x 8 block of 16-byte chunks held by eight consecutive lanes (lane l: row l, chunks 0..7): afterwards
+// lane l holds chunk l of rows 0..7, with which one warp-wide access touches four 128-byte lines instead of 32.
+__device__ __forceinline__ void transpose_chunks(uint4 (&c)[8], int lane) {
+    #pragma unroll
+    for (int k = 1; k < 8; k <<= 1) {
+        const bool up = (lane & k) != 0;
+        #pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i & k) continue;
+            uint4 t = up ? c[i] : c[i | k];
+            t.x = __shfl_xor_sync(0xffffffffu, t.x, k);
+            t.y = __shfl_xor_sync(0xffffffffu, t.y, k);
+            t.z = __shfl_xor_sync(0xffffffffu, t.z, k);
+            t.w = __shfl_xor_sync(0xffffffffu, t.w, k);
+            if (up) c[i] = t; else c[i | k] = t;
+        }
+    }
 }
 
 template <int V> struct IntTag { static constexpr int value = V; };
@@ -1319,6 +1318,28 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             }
         }
         (void)pk_pre;
+        // TURN_IO: the epilogue operands, chunk lane % 8 of rows turn_row0 ... + 7, on their way meanwhile
+        const int turn_row0 = own0 + (warp & 3) * 32 + (lane & 24);
+        const int turn_col0 = (grp * NSPLIT + sp) * (DPAD / (NSPLIT * NG));
+        constexpr int TURN_N = CFG::TURN_IO ? 8 : 1, TURN_OPER = CFG::TURN_IO && MODE == kBwd2Row ? 8 : 1;
+        uint4 turn0[TURN_N], turn1[TURN_N], turn_pk[2][TURN_OPER];       // dQ / first result, out / second result, pk
+        (void)turn0; (void)turn1; (void)turn_pk; (void)turn_row0; (void)turn_col0;
+        if constexpr (CFG::TURN_IO && MODE == kBwd2Row) {
+            const int col = turn_col0 + (lane & 7) * 8, col_pk = turn_col0 + (lane & 7) * 4;
+            const uint16_t* g_out = static_cast<const uint16_t*>(p.out) + (long long)batch * p.out_sb + (long long)head * p.out_sh + col;
+            const uint16_t* g_dq = static_cast<const uint16_t*>(p.dQ) + (long long)batch * p.dQ_sb + (long long)head * p.dQ_sh + col;
+            const float* g_pk = p.pk + ((long long)batch * p.Hq + head) * p.Nq * p.D + col_pk;
+            #pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const long long r = turn_row0 + i;
+                const bool ok = r < n_own;
+                const uint4 zero = make_uint4(0, 0, 0, 0);
+                turn0[i] = ok && col < p.D ? __ldg(reinterpret_cast<const uint4*>(g_dq + r * p.dQ_sn)) : zero;
+                turn1[i] = ok && col < p.D ? __ldg(reinterpret_cast<const uint4*>(g_out + r * p.out_sn)) : zero;
+                turn_pk[0][i] = ok && col_pk < p.D ? __ldg(reinterpret_cast<const uint4*>(g_pk + r * p.D)) : zero;
+                turn_pk[1][i] = ok && col_pk + 32 < p.D ? __ldg(reinterpret_cast<const uint4*>(g_pk + r * p.D + 32)) : zero;
+            }
+        }
         float alpha = 0.f, ecirc = 0.f;
         if constexpr (MODE == kBwd2Row) {
             // Every pointwise thread of my row holds a partial sum.  The exchange buffer alternates between items
@@ -1344,7 +1365,6 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             constexpr int DC = DPAD / (NSPLIT * NG);    // output columns per pointwise thread
             constexpr int NCH = DC / 16;
             const int res_heads = COL ? p.Hkv : p.Hq;
-            const long long res_off = (((long long)batch * res_heads + head) * n_own + own_idx) * p.D;
             // All of my accumulator columns come out of tensor memory first (warp-wide loads), so that
             // the MMA warp may start overwriting them for the next item while I combine and store.
             // (With more than two 16-column chunks per thread that would cost too many registers: then
@@ -1380,7 +1400,29 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                                  pack2<BF16>(v[8 * i + 4], v[8 * i + 5]), pack2<BF16>(v[8 * i + 6], v[8 * i + 7]));
                 }
             };
-            (void)stage16; (void)res_off;
+            (void)stage16; (void)res_heads;
+            // 16 columns of my row, the c-th of this thread on, as two chunks
+            auto pack_chunks = [&](uint4 (&dst)[TURN_N], int c, const float* v) {
+                #pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    dst[c / 8 + i] = make_uint4(pack2<BF16>(v[8 * i], v[8 * i + 1]), pack2<BF16>(v[8 * i + 2], v[8 * i + 3]),
+                                                pack2<BF16>(v[8 * i + 4], v[8 * i + 5]), pack2<BF16>(v[8 * i + 6], v[8 * i + 7]));
+            };
+            (void)pack_chunks;
+            // rows turned around by transpose_chunks, as 16-byte chunks at column offset `col` of my eight rows
+            auto store_turned = [&](auto* base, const uint4 (&c)[8], int col) {
+                auto* dst = base + (((long long)batch * res_heads + head) * n_own + turn_row0) * p.D + col;
+                #pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (turn_row0 + i < n_own && col < p.D) *reinterpret_cast<uint4*>(dst + (long long)i * p.D) = c[i];
+            };
+            (void)store_turned;
+            if constexpr (CFG::TURN_IO && MODE == kBwd2Row) {
+                transpose_chunks(turn0, lane);           // now my own row's 64 columns
+                transpose_chunks(turn1, lane);
+                transpose_chunks(turn_pk[0], lane);
+                transpose_chunks(turn_pk[1], lane);
+            }
             #pragma unroll
             for (int c = 0; c < DC; c += 16) {
                 const int col = (grp * NSPLIT + sp) * DC + c;
@@ -1409,11 +1451,6 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                             for (int i = 0; i < 4; ++i)
                                 st_shared_v4(base + sw128_offset(row, (col % 32) / 4 + i), __float_as_uint(a1[4 * i]), __float_as_uint(a1[4 * i + 1]),
                                              __float_as_uint(a1[4 * i + 2]), __float_as_uint(a1[4 * i + 3]));
-                        } else if (own_ok) {
-                            float4* dst = reinterpret_cast<float4*>(p.pk + res_off + col);
-                            #pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                dst[i] = make_float4(a1[4 * i], a1[4 * i + 1], a1[4 * i + 2], a1[4 * i + 3]);
                         }
                     }
                 } else if constexpr (COL) {
@@ -1422,12 +1459,12 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                     if constexpr (CFG::STAGED_OUT) {
                         stage16(io_out, col, a0);
                         stage16(io_out + CFG::OWN_TILE_BYTES, col, a1);
-                    } else if (own_ok) {
-                        store16_from_float<BF16>(p.res0, res_off + col, a0);
-                        store16_from_float<BF16>(p.res1, res_off + col, a1);
+                    } else {
+                        pack_chunks(turn0, c, a0);
+                        pack_chunks(turn1, c, a1);
                     }
                 } else {
-                    if (!own_ok) continue;
+                    if (CFG::STAGED_IO && !own_ok) continue;
                     // accumulators: a0 = P uV + (P*F) V, a1 = (P*T) K + dS uK;  PK comes from the first backward
                     float o[16], g[16], pkv[16];
                     if constexpr (CFG::STAGED_IO) {
@@ -1441,16 +1478,17 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                             unpack8_as_float<BF16>(ld_shared_v4(io_dq + off), g + 8 * i);
                         }
                     } else {
-                        const float4* src = reinterpret_cast<const float4*>(p.pk + res_off + col);
                         #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            const float4 t = src[i];
-                            pkv[4 * i] = t.x; pkv[4 * i + 1] = t.y; pkv[4 * i + 2] = t.z; pkv[4 * i + 3] = t.w;
+                            const uint4 t = turn_pk[c / 32][(c % 32) / 4 + i];
+                            pkv[4 * i] = __uint_as_float(t.x); pkv[4 * i + 1] = __uint_as_float(t.y);
+                            pkv[4 * i + 2] = __uint_as_float(t.z); pkv[4 * i + 3] = __uint_as_float(t.w);
                         }
-                        load16_as_float<BF16>(p.out, (long long)batch * p.out_sb + (long long)head * p.out_sh +
-                                                         (long long)own_idx * p.out_sn + col, o);
-                        load16_as_float<BF16>(p.dQ, (long long)batch * p.dQ_sb + (long long)head * p.dQ_sh +
-                                                        (long long)own_idx * p.dQ_sn + col, g);
+                        #pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            unpack8_as_float<BF16>(turn1[c / 8 + i], o + 8 * i);
+                            unpack8_as_float<BF16>(turn0[c / 8 + i], g + 8 * i);
+                        }
                     }
                     #pragma unroll
                     for (int i = 0; i < 16; ++i) {
@@ -1463,9 +1501,27 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                         stage16(io_dq, col, a0);
                         stage16(io_out, col, a1);
                     } else {
-                        store16_from_float<BF16>(p.res0, res_off + col, a0);
-                        store16_from_float<BF16>(p.res1, res_off + col, a1);
+                        pack_chunks(turn0, c, a0);
+                        pack_chunks(turn1, c, a1);
                     }
+                }
+            }
+            if constexpr (CFG::TURN_IO) {
+                transpose_chunks(turn0, lane);
+                transpose_chunks(turn1, lane);
+                store_turned(static_cast<uint16_t*>(p.res0), turn0, turn_col0 + (lane & 7) * 8);
+                store_turned(static_cast<uint16_t*>(p.res1), turn1, turn_col0 + (lane & 7) * 8);
+            }
+            if constexpr (CFG::TURN_PK) {
+                if (p.pk) {
+                    uint4 t[8];
+                    #pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float* a1 = acc1[EARLY ? i / 4 : 0] + 4 * (i % 4);
+                        t[i] = make_uint4(__float_as_uint(a1[0]), __float_as_uint(a1[1]), __float_as_uint(a1[2]), __float_as_uint(a1[3]));
+                    }
+                    transpose_chunks(t, lane);
+                    store_turned(p.pk, t, turn_col0 + (lane & 7) * 4);
                 }
             }
         }
