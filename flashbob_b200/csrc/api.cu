@@ -124,7 +124,7 @@ static int launch_sweep(const bob_sm100_geom* g, SweepParams& prm, const TensorA
         int rc = build(own_tensor<MODE>(i), 128);
         if (rc) return rc;
     }
-    if (CFG::OWN_OUT) {
+    if (CFG::OWN_OUT && !prm.out) {
         int rc = build(kTOUT, 128);
         if (rc) return rc;
     }
@@ -467,6 +467,9 @@ extern "C" int bob_sm100_bwd1(const bob_sm100_geom* g, const void* q, const void
     p.delta = delta;
     p.pk = pk;
     p.res0 = dQ;
+    int64_t sn = g->out_strides[2], sh = g->out_strides[1], sb = g->out_strides[0];
+    if (fit_strides(g->D, g->Nq, g->Hq, g->B, sn, sh, sb, TileType::kF16))      // an expanded `out`: no tile of it
+        set_strided(p.out, p.out_sb, p.out_sh, p.out_sn, out, g->out_strides);
     rc = dispatch_dtype<kBwd1Row>(g, p, t, s, 0);   // dQ and delta
     if (rc) return rc;
     p.res0 = dK;

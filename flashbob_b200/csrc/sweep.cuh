@@ -59,7 +59,7 @@ struct SweepParams {
     float scale;
     int has_uq, has_uk, has_uv;   // 0 = that tangent is undefined (treated as zero, products skipped)
     // global tensors read with plain loads (element strides: batch, head, row; unit head-dim stride)
-    const void* out;  long long out_sb, out_sh, out_sn;
+    const void* out;  long long out_sb, out_sh, out_sn;    // first backward: only where a tile cannot be addressed (zero strides)
     const void* dQ;   long long dQ_sb, dQ_sh, dQ_sn;
     // fp32 row statistics, contiguous [B, Hq, Nq]
     float* lse;       // natural log
@@ -369,6 +369,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
     }
 
     auto has_tensor = [&](int t) {
+        if (CFG::OWN_OUT && t == kTOUT) return p.out == nullptr;     // otherwise read with plain loads
         return t == kTUQ ? has_uq : (t == kTUK ? has_uk : (t == kTUV ? has_uv : true));
     };
 
@@ -520,7 +521,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                 break;
             }
             if (lane == 0) {
-                uint32_t own_bytes = CFG::OWN_OUT ? CFG::OWN_TILE_BYTES : 0;
+                uint32_t own_bytes = CFG::OWN_OUT && has_tensor(kTOUT) ? CFG::OWN_TILE_BYTES : 0;
                 #pragma unroll
                 for (int i = 0; i < MT::NOWN; ++i)
                     if (has_tensor(own_tensor<MODE>(i))) own_bytes += CFG::OWN_TILE_BYTES;
@@ -915,7 +916,12 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                     const int ch = part * CH + c;
                     const uint32_t off = (ch / 8) * (128 * 128) + sw128_offset(row, ch % 8);
                     float a[8], b[8];
-                    unpack8_as_float<BF16>(ld_shared_v4(t_out + off), a);
+                    uint4 w = make_uint4(0, 0, 0, 0);
+                    if (!p.out) w = ld_shared_v4(t_out + off);
+                    else if (own_ok && ch * 8 < p.D)
+                        w = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.out) + (long long)batch * p.out_sb +
+                                                            (long long)head * p.out_sh + (long long)own_idx * p.out_sn + ch * 8);
+                    unpack8_as_float<BF16>(w, a);
                     unpack8_as_float<BF16>(ld_shared_v4(t_do + off), b);
                     #pragma unroll
                     for (int i = 0; i < 8; ++i) sum = fmaf(a[i], b[i], sum);
