@@ -200,6 +200,7 @@ struct SweepConfig {
     static constexpr int NSLOT = SLOT_ROOM >= MAX_SLOTS ? MAX_SLOTS : SLOT_ROOM;
     static_assert(SPLIT_KV ? NSLOT >= 2 * NG : NSLOT > NG, "score products run up to NG tiles ahead");
     static_assert(NG * SLOTS_PER_TILE <= NSLOT, "a group's step through the ring wraps at most once");
+    static_assert(!ALIAS || 2 * SLOTS_PER_TILE <= NSLOT, "two tiles on, a tile's slot is at the earliest in use again");
     static constexpr int OFF_OWN = 0;
     static constexpr int OFF_OTH = OFF_OWN + OWN_TILES * OWN_TILE_BYTES;
     static constexpr int OFF_IO = OFF_OTH + NSLOT * SLOT_BYTES;                 // staged results / epilogue operands
@@ -700,8 +701,10 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             using NS1 = IntTag<1>;
             using NS2 = IntTag<2>;
             uint32_t free_par = 0;               // !ALIAS: bit g = parity of group g's next "scores read" wait
-            int last_s0 = -1, last_s1 = -1;      // ALIAS: slot and parity of each group's last tile (-1: none yet)
-            int last_p0 = 0, last_p1 = 0;
+            // ALIAS: each group's last tile - its slot, parity and number (-1: none yet) - and the newest tile whose
+            // products are known to have finished.
+            int last_s0 = 0, last_s1 = 0, last_p0 = 0, last_p1 = 0, last_n0 = -1, last_n1 = -1;
+            int n_sc = 0, done_n = -1;
             for (int k_item = 0;; ++k_item) {
                 const int item = follow_ring_alone(k_item);
                 if (item == -2) give_up(kStatusTimeoutMma);
@@ -722,9 +725,18 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                     wait_alone(bar_full(s), par, kStatusTimeoutMma);
                     BOB_TR(1)
                     if constexpr (ALIAS) {
-                        // the group's operands sit in its score columns until its output products have read them
-                        const int ls = g ? last_s1 : last_s0;
-                        if (ls >= 0) wait_alone(bar_empty(ls), g ? last_p1 : last_p0, kStatusTimeoutMma);
+                        // The group's operands sit in its score columns until its output products have read them.
+                        // Products finish in the order of the tiles, so a tile up to done_n needs no wait, and must have
+                        // none: after an item with an odd number of tiles a group's last tile is three or more back, its
+                        // slot may have been filled and emptied once more, and the parity would then mean a
+                        // phase that only tiles yet to be issued can complete.  Where the wait is taken, the other group
+                        // has had at most one tile since (with a second one, that one's wait raised done_n), so
+                        // the slot's next tile is not issued yet.
+                        const int ln = g ? last_n1 : last_n0;
+                        if (ln > done_n) {
+                            wait_alone(bar_empty(g ? last_s1 : last_s0), g ? last_p1 : last_p0, kStatusTimeoutMma);
+                            done_n = ln;
+                        }
                     } else {
                         wait_alone(bar_sc_empty(g), ((free_par >> g) & 1u) ^ 1u, kStatusTimeoutMma);
                         free_par ^= 1u << g;
@@ -761,7 +773,8 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
                     BOB_TR(3)
                     int vs = s + SPT - 1, vp = par;                   // the tile's last slot (forward: V's)
                     if (SPT == 2 && vs == NSLOT) { vs = 0; vp ^= 1; }
-                    if (g) { last_s1 = vs; last_p1 = vp; } else { last_s0 = vs; last_p0 = vp; }
+                    if (g) { last_s1 = vs; last_p1 = vp; last_n1 = n_sc; } else { last_s0 = vs; last_p0 = vp; last_n0 = n_sc; }
+                    ++n_sc;
                     if constexpr (NG == 2) g ^= 1;
                     s += SPT;
                     if (s >= NSLOT) { s -= NSLOT; par ^= 1; }
@@ -871,7 +884,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             pw_all_phase ^= 1u;
         };
         int s = 0, par = 0;                      // slot of the item's next tile, parity of its use
-        int last_s = -1, last_par = 0;           // !ALIAS: my group's last tile, whose products must have read its operands
+        int last_s = -1, last_par = 0;           // !ALIAS: my group's last tile of this item, whose products must have read its operands
         uint32_t sc_par = 0;                     // parity of my group's next scores
         int n_live = 0;                          // items with at least one tile finished so far
         int n_done = 0;                          // items finished so far, with or without tiles
@@ -1363,6 +1376,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
             if (grp == 0 && sp == 0 && own_ok) { p.alpha[row_stat] = alpha; p.ecirc[row_stat] = ecirc; }
         }
         if (total > 0) wait(bar_done, n_live & 1, kStatusTimeoutPw);
+        last_s = -1;                                 // all products have finished; by the group's next tile the slot may be in use again
         tc_fence_after_sync();
         // the previous item's results have left the staging buffer
         if constexpr (CFG::STAGED_OUT) wait(bar_io_free, (n_done & 1) ^ 1, kStatusTimeoutPw);
