@@ -1361,18 +1361,21 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
         }
         float alpha = 0.f, ecirc = 0.f;
         if constexpr (MODE == kBwd2Row) {
-            // Every pointwise thread of my row holds a partial sum.  The exchange buffer alternates between items
-            // where there is room for two; elsewhere it is written only once the item's products have
-            // finished, which they cannot before every warp has left the previous item's epilogue.
+            // Every pointwise thread of my row holds a partial sum.  The exchange buffer alternates between items with
+            // tiles where there is room for two; elsewhere it is written only once the item's products have finished,
+            // which they cannot before every warp has left the epilogue of the previous item with tiles.  An item
+            // without tiles has no sums to exchange, and no products to wait for before it could write the buffer.
             constexpr int NPART = NG * NSPLIT;
-            float* xb = red_buf + (CFG::RED_COPIES == 2 ? (n_done & 1) * (2 * NPART * 128) : 0);
-            if (CFG::RED_COPIES == 1 && total > 0) wait(bar_done, n_live & 1, kStatusTimeoutPw);
-            xb[(grp * NSPLIT + sp) * 128 + row] = acc_a.x + acc_a.y;
-            xb[(NPART + grp * NSPLIT + sp) * 128 + row] = acc_b.x + acc_b.y;
+            if (total > 0) {
+                float* xb = red_buf + (CFG::RED_COPIES == 2 ? (n_live & 1) * (2 * NPART * 128) : 0);
+                if (CFG::RED_COPIES == 1) wait(bar_done, n_live & 1, kStatusTimeoutPw);
+                xb[(grp * NSPLIT + sp) * 128 + row] = acc_a.x + acc_a.y;
+                xb[(NPART + grp * NSPLIT + sp) * 128 + row] = acc_b.x + acc_b.y;
+                all_sync();
+                #pragma unroll
+                for (int k = 0; k < NPART; ++k) { alpha += xb[k * 128 + row]; ecirc += xb[(NPART + k) * 128 + row]; }
+            }
             if constexpr (CFG::STAGED_IO) wait(bar_io_full, n_done & 1, kStatusTimeoutPw);   // the IO warp has staged out, dQ
-            all_sync();
-            #pragma unroll
-            for (int k = 0; k < NPART; ++k) { alpha += xb[k * 128 + row]; ecirc += xb[(NPART + k) * 128 + row]; }
             if (grp == 0 && sp == 0 && own_ok) { p.alpha[row_stat] = alpha; p.ecirc[row_stat] = ecirc; }
         }
         if (total > 0) wait(bar_done, n_live & 1, kStatusTimeoutPw);

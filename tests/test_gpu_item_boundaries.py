@@ -46,3 +46,10 @@ def _check(B, H, Nq, Nk, D, dtype, repeats, second=True, **mask):
 ])
 def test_items_with_an_odd_number_of_tiles(D, Nq, Nk, mask):
     _check(3, 64, Nq, Nk, D, torch.bfloat16, 20, second=False, **mask)
+
+
+@pytest.mark.parametrize("D", [128, 80, 64])
+def test_items_without_keys_between_items_with_keys(D):
+    """Keys start 300 positions after the queries: the first own tiles of every head attend to nothing, and a CTA takes
+    such items after others with the row sums of the second backward in its exchange buffer."""
+    _check(3, 64, 640, 384, D, torch.bfloat16, 20, is_causal=True, q_offset=0, k_offset=300)
