@@ -19,6 +19,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <cmath>
 #include <optional>
@@ -248,10 +249,11 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const Mask& m) {
 bool is_int(PyObject* o) { return PyLong_CheckExact(o); }       // a bool is a subclass: not exact
 
 // The argument checks of sdpa_bob in their common, valid form.  Anything else - a CPU tensor, an int-like
-// that is no int, a grouped call with a window, an invalid shape - is left to the Python checks, which
-// raise or resolve it; they are the one statement of what is allowed.
+// that is no int, a grouped call with a window, an invalid shape, a call that torch.jit.trace records - is left
+// to the Python side, which raises or resolves it; its checks are the one statement of what is allowed.
 bool common_call(const Tensor& q, const Tensor& k, const Tensor& v, PyObject* causal, PyObject* scale, PyObject* window,
                  PyObject* q_offset, PyObject* k_offset, Mask& m) {
+    if (torch::jit::tracer::isTracing()) return false;
     const auto type = q.scalar_type();
     if (!q.is_cuda() || q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || (type != at::kHalf && type != at::kBFloat16)) return false;
     if (k.scalar_type() != type || v.scalar_type() != type || k.device() != q.device() || v.device() != q.device()) return false;

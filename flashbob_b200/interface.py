@@ -11,6 +11,9 @@ protocol (reference: src/bob/sdpa.py:239-368), whose nodes are native (csrc/torc
     node over (q, k, v, dO) whose backward is the second backward, returning gradients for those;
   * undefined incoming tangents stay undefined and switch off the products they would feed.
 
+While `torch.jit.trace` records, the same chain runs as Python autograd functions: the tracer records such a function
+as an operation of its graph, but takes the result of a native node for a constant.
+
 CUDA tensors always go through the CUDA library: there is no fallback, a missing library raises.
 CPU tensors take PyTorch's math attention with stock autograd, exactly as the reference's CPU
 route does (reference: src/bob/sdpa.py:437-465).
@@ -23,6 +26,7 @@ import numbers
 import operator as _operator
 
 import torch
+from torch.autograd import Function
 
 from . import _native, ops
 
@@ -159,6 +163,57 @@ def _cpu_math_attention(q, k, v, *, is_causal, window, q_offset, k_offset, scale
 
 
 # --------------------------------------------------------------------------------------
+# autograd chain under torch.jit.trace
+# --------------------------------------------------------------------------------------
+class BoBSecondOrder(Function):
+    """First backward as a differentiable function of (q, k, v, dO); its backward is the second backward."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, dO, out, lse, geom):
+        ctx.set_materialize_grads(False)
+        dQ, dK, dV, delta, pk = ops.attention_first_backward(q, k, v, out, lse, dO, **geom)
+        ctx.save_for_backward(q, k, v, out, lse, dO, dQ, delta, pk)
+        ctx.geom = geom
+        return dQ, dK, dV
+
+    @staticmethod
+    def backward(ctx, uQ, uK, uV):
+        q, k, v, out, lse, dO, dQ, delta, pk = ctx.saved_tensors
+        if uQ is None and uK is None and uV is None:
+            return (None,) * 7
+        return (*ops.attention_second_backward(q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV, **ctx.geom), None, None, None)
+
+
+class SDPAWithBoB(Function):
+    """Attention forward whose backward is itself differentiable once more.  The mask arrives as numbers (a
+    traced shape makes an offset a zero-dimensional tensor): the recorded operation keeps them as its constants."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, q_offset, k_offset, is_causal, window_size, scale):
+        ctx.set_materialize_grads(False)
+        geom = dict(is_causal=is_causal, window_size=window_size, q_offset=int(q_offset), k_offset=int(k_offset), scale=scale)
+        out, lse = ops.attention_forward(q, k, v, **geom)
+        if torch.jit.is_tracing():                  # the tracer takes over results that it has seen being made
+            known = torch.empty_like(q)
+            known.data = out
+            out = known
+        ctx.save_for_backward(q, k, v, out, lse)
+        ctx.geom = geom
+        return out
+
+    @staticmethod
+    def backward(ctx, dO):
+        if dO is None:
+            return (None,) * 8
+        q, k, v, out, lse = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            grads = BoBSecondOrder.apply(q, k, v, dO, out, lse, ctx.geom)
+        else:
+            grads = ops.attention_first_backward(q, k, v, out, lse, dO, for_second_order=False, **ctx.geom)[:3]
+        return (*grads, None, None, None, None, None)
+
+
+# --------------------------------------------------------------------------------------
 # public operator
 # --------------------------------------------------------------------------------------
 def sdpa_bob(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, is_causal: bool = False,
@@ -200,4 +255,6 @@ def sdpa_bob(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, is_causal: bo
     if not q.is_cuda:
         return _cpu_math_attention(q, k, v, is_causal=is_causal, window=window, q_offset=q_off,
                                    k_offset=k_off, scale=scale, rectangular=rectangular)
+    if torch.jit.is_tracing():
+        return SDPAWithBoB.apply(q, k, v, q_off, k_off, is_causal, window, scale)
     return _native.load().sdpa(q, k, v, is_causal, window, q_off, k_off, scale, ops._CHECK_STATUS)
