@@ -201,6 +201,9 @@ struct SdpaNode : Node {
         if (!dO.defined()) return variable_list(3);
         const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), out_ = out.unpack(shared_from_this()), lse_ = lse.unpack();
         const bool record = torch::autograd::compute_requires_grad(q_, k_, v_, dO);
+        // a graph that is kept would hold a derivative from which the tangent's term is missing
+        TORCH_CHECK_NOT_IMPLEMENTED(!record || !dO._fw_grad(0).defined(), "forward-mode AD is unsupported; differentiate with "
+                                    "reverse mode (torch.autograd.grad twice) instead");
         First r;
         {
             Untracked untracked;

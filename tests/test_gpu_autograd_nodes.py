@@ -2,6 +2,7 @@
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fwAD
 
 import bob
 
@@ -46,3 +47,12 @@ def test_a_traced_call_computes_with_its_inputs(nq, nk, kw):
     traced = torch.jit.trace(op, example)
     for _ in range(3):                          # the first runs profile, the later ones run optimised
         _same(_step(traced, leaves, dO, bars), _step(op, leaves, dO, bars))
+
+
+def test_a_forward_mode_tangent_of_the_output_gradient_is_refused_where_a_graph_is_kept():
+    leaves, dO, _ = _inputs(0)
+    out = causal(*leaves)
+    with fwAD.dual_level():
+        weight = fwAD.make_dual(dO.detach(), torch.ones_like(dO))
+        with pytest.raises(NotImplementedError):
+            torch.autograd.grad((out * weight).sum(), leaves, create_graph=True)
