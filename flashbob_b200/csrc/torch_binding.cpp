@@ -57,7 +57,7 @@ struct Mask {
     bool causal = false;
     int window = 0;
     int64_t q_offset = 0, k_offset = 0;
-    double scale = 0;                      // 0: 1 / sqrt(D)
+    std::optional<double> scale;           // none: 1 / sqrt(D)
     bool check_status = false;             // wait for the stream after each stage and read its status word
 };
 
@@ -83,7 +83,7 @@ bob_sm100_geom geometry(const Tensor& q, const Tensor& k, const Mask& m) {
     g.device = q.device().index();
     g.q_offset = m.q_offset;
     g.k_offset = m.k_offset;
-    g.scale = static_cast<float>(m.scale > 0 ? m.scale : 1.0 / std::sqrt(static_cast<double>(g.D)));
+    g.scale = static_cast<float>(m.scale ? *m.scale : 1.0 / std::sqrt(static_cast<double>(g.D)));
     return g;
 }
 
@@ -289,8 +289,9 @@ bool common_call(const Tensor& q, const Tensor& k, const Tensor& v, PyObject* ca
     if (group > 1 && (rectangular || w > 0 || type != at::kBFloat16 || group > 32)) return false;
     if (scale != Py_None) {
         if (!PyFloat_CheckExact(scale)) return false;
+        const float s = static_cast<float>(PyFloat_AS_DOUBLE(scale));
+        if (!(s > 0) || !std::isfinite(s)) return false;
         m.scale = PyFloat_AS_DOUBLE(scale);
-        if (!(m.scale > 0) || !std::isfinite(static_cast<float>(m.scale)) || !(static_cast<float>(m.scale) > 0)) return false;
     }
     return true;
 }

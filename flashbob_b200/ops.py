@@ -57,6 +57,11 @@ def _geom(q, k, *, is_causal, window_size, q_offset, k_offset, scale) -> _lib.Ge
     return g
 
 
+def _mask(is_causal, window_size, q_offset, k_offset, scale):
+    """The mask arguments of the native calls, converted as `_geom` converts them; the C ABI refuses what is out of range."""
+    return (bool(is_causal), int(window_size), int(q_offset), int(k_offset), None if scale is None else float(scale), _CHECK_STATUS)
+
+
 def check_device_status(device=None) -> None:
     """Raise if any libbob_sm100 kernel on `device` gave up on a bounded wait since the last check.
     Non-blocking; call it after a synchronisation point (for instance at the end of a training step)
@@ -80,7 +85,7 @@ def _require_cuda_16bit(*tensors) -> None:
 def attention_forward(q, k, v, *, is_causal, window_size, q_offset, k_offset, scale):
     """out [B,Hq,Nq,D] (input dtype) and natural-log lse [B,Hq,Nq] (fp32)."""
     _require_cuda_16bit(q, k, v)
-    return _native.load().forward(q, k, v, bool(is_causal), window_size, q_offset, k_offset, scale, _CHECK_STATUS)
+    return _native.load().forward(q, k, v, *_mask(is_causal, window_size, q_offset, k_offset, scale))
 
 
 def attention_first_backward(q, k, v, out, lse, dO, *, is_causal, window_size, q_offset, k_offset,
@@ -88,13 +93,12 @@ def attention_first_backward(q, k, v, out, lse, dO, *, is_causal, window_size, q
     """dQ, dK, dV (input dtype, contiguous), delta = rowsum(dO*out) [B,Hq,Nq] (fp32) and, when
     `for_second_order`, pk = softmax(S) K [B,Hq,Nq,D] (fp32) for the second backward (else None)."""
     _require_cuda_16bit(q, k, v, out, dO)
-    return _native.load().first_backward(q, k, v, out, lse, dO, bool(is_causal), window_size, q_offset, k_offset, scale,
-                                         _CHECK_STATUS, for_second_order)
+    return _native.load().first_backward(q, k, v, out, lse, dO, *_mask(is_causal, window_size, q_offset, k_offset, scale), for_second_order)
 
 
 def attention_second_backward(q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV, *, is_causal,
                               window_size, q_offset, k_offset, scale):
     """Qbar, Kbar, Vbar, dObar (input dtype, contiguous).  uQ/uK/uV may be None."""
     _require_cuda_16bit(q, k, v, out, dO, dQ, uQ, uK, uV)
-    return _native.load().second_backward(q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV, bool(is_causal), window_size,
-                                          q_offset, k_offset, scale, _CHECK_STATUS)
+    return _native.load().second_backward(q, k, v, out, lse, delta, pk, dO, dQ, uQ, uK, uV,
+                                          *_mask(is_causal, window_size, q_offset, k_offset, scale))
