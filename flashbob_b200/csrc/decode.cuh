@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) decode_kernel(const __grid_
     __syncthreads();
     auto finish = [&](int i, int col, float value, float ref, float sum) {       // row i, column col of the result
         const long long row = (long long)unit * p.Nq + i;
-        const float r = sum > 0.f ? value / sum : 0.f;
+        // no key: zero.  An infinite score makes the sum NaN, and the row with it.
+        const float r = sum > 0.f ? value / sum : (ref == INFINITY ? sum : 0.f);
         p.out[row * p.D + col] = static_cast<uint16_t>(pack2<BF16>(r, 0.f));
         if (col == 0) p.lse[row] = sum > 0.f ? (ref + log2f(sum)) * kLn2 : -INFINITY;
     };
