@@ -28,7 +28,7 @@ class Geom(ctypes.Structure):
         ("dtype", ctypes.c_int32), ("is_causal", ctypes.c_int32), ("window", ctypes.c_int32),
         ("device", ctypes.c_int32),
         ("q_offset", ctypes.c_int64), ("k_offset", ctypes.c_int64),
-        ("scale", ctypes.c_float), ("reserved", ctypes.c_int32),
+        ("scale", ctypes.c_float), ("flags", ctypes.c_int32),
         ("q_strides", ctypes.c_int64 * 3), ("k_strides", ctypes.c_int64 * 3),
         ("v_strides", ctypes.c_int64 * 3), ("out_strides", ctypes.c_int64 * 3),
         ("do_strides", ctypes.c_int64 * 3), ("dq_strides", ctypes.c_int64 * 3),

@@ -257,8 +257,9 @@ static void set_strided(const void*& dst, long long& sb, long long& sh, long lon
 
 // ---- forward with a few query rows ------------------------------------------------------------------
 // Up to kDecodeRows query rows per head go to decode_kernel whatever the number of keys: the sweep kernel would
-// do the work of 128 rows for them.  A head's keys are divided until kDecodeCtas CTAs are there (two are resident
-// per SM), but not below one round of a CTA's warps.
+// do the work of 128 rows for them.  Where the caller's workspace is sized for it (BOB_SM100_SPLIT_KEYS), a head's keys
+// are divided until kDecodeCtas CTAs are there (two are resident per SM), but not below one round of a CTA's warps.
+// (The number is B200's and not asked of the device, so that the workspace's size depends on the geometry alone.)
 constexpr int kDecodeCtas = 4 * 148;
 struct DecodePlan { int k_lo, k_hi, splits, split_keys; size_t acc_offset, bytes; };     // offsets in the workspace
 
@@ -276,7 +277,8 @@ static DecodePlan decode_plan(const bob_sm100_geom* g) {
     const int dpad = g->D <= 32 ? 32 : (g->D <= 64 ? 64 : 128);
     const int64_t round = decode_round(dpad, g->Nq), rounds = std::max<int64_t>(1, (hi - lo + round - 1) / round);
     const int64_t heads = (int64_t)g->B * g->Hq;
-    const int64_t want = std::min<int64_t>({kDecodeMaxSplits, rounds, std::max<int64_t>(1, kDecodeCtas / heads)});
+    const int64_t want = !(g->flags & BOB_SM100_SPLIT_KEYS) ? 1
+                                                            : std::min<int64_t>({kDecodeMaxSplits, rounds, std::max<int64_t>(1, kDecodeCtas / heads)});
     const int64_t per = (rounds + want - 1) / want;
     d.split_keys = (int)(per * round);
     d.splits = (int)((rounds + per - 1) / per);

@@ -81,6 +81,7 @@ bob_sm100_geom geometry(const Tensor& q, const Tensor& k, const Mask& m) {
     g.is_causal = m.causal;
     g.window = m.window;
     g.device = q.device().index();
+    g.flags = BOB_SM100_SPLIT_KEYS;        // (every workspace below is sized for its own call)
     g.q_offset = m.q_offset;
     g.k_offset = m.k_offset;
     g.scale = static_cast<float>(m.scale ? *m.scale : 1.0 / std::sqrt(static_cast<double>(g.D)));

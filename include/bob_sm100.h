@@ -31,8 +31,10 @@
  *     lse and delta 4-byte aligned (checked on the host: error -10).
  *   - No entry point allocates or frees device memory (except bob_sm100_selftest's caller-owned
  *     buffers, which are arguments too).  Scratch is passed in as `workspace`, at least
- *     bob_sm100_workspace_bytes(stage, geom) bytes, 256-byte aligned.  Its first word is a
- *     status word that the call clears and a kernel sets if a bounded wait ran out.
+ *     bob_sm100_workspace_bytes(stage, geom) bytes, 256-byte aligned.  That is 256 for the forward
+ *     (unless geom->flags has BOB_SM100_SPLIT_KEYS) and the first backward, and grows with B * Hq * Nq for the
+ *     second backward.  Its first word is a status word that the call clears and a kernel sets if a bounded
+ *     wait ran out.
  *   - Work is enqueued on `stream` (a cudaStream_t; NULL = legacy default stream) and the call
  *     returns without synchronising.  Calls are re-entrant; concurrent calls need distinct
  *     workspaces.
@@ -51,6 +53,11 @@ extern "C" {
 
 enum { BOB_SM100_FP16 = 0, BOB_SM100_BF16 = 1 };
 enum { BOB_SM100_STAGE_FWD = 0, BOB_SM100_STAGE_BWD1 = 1, BOB_SM100_STAGE_BWD2 = 2 };
+/* geom->flags: the forward's workspace is as large as bob_sm100_workspace_bytes says for this very geometry (sizes,
+ * mask and offsets), so a forward with at most four query rows may divide a head's keys between several CTAs and
+ * park their parts there.  Without it the forward's workspace is 256 bytes for every geometry, and one CTA reads all
+ * keys of a head of such a call. */
+enum { BOB_SM100_SPLIT_KEYS = 1 };
 
 typedef struct bob_sm100_geom {
     int32_t B, Hq, Hkv, Nq, Nk, D;
@@ -61,7 +68,7 @@ typedef struct bob_sm100_geom {
     int64_t q_offset;    /* absolute position of query row 0 */
     int64_t k_offset;    /* absolute position of key row 0 */
     float scale;         /* softmax scale, finite and > 0 */
-    int32_t reserved;
+    int32_t flags;       /* 0, or BOB_SM100_SPLIT_KEYS */
     /* element strides (batch, head, row) of each input tensor */
     int64_t q_strides[3];
     int64_t k_strides[3];
