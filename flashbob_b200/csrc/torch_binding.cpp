@@ -170,6 +170,10 @@ struct Untracked {
     at::AutoDispatchBelowADInplaceOrView below;
 };
 
+// deleteNode frees a graph node by node; a plain destructor would free a node's predecessors inside its own, one
+// stack frame deeper for each of a chain of calls.
+template <class N> std::shared_ptr<N> make_node() { return std::shared_ptr<N>(new N(), torch::autograd::deleteNode); }
+
 // First backward as a differentiable function of (q, k, v, dO): its gradient is the second backward.
 struct SecondOrderNode : Node {
     Mask mask;
@@ -212,7 +216,7 @@ struct SdpaNode : Node {
             r = run_first(q_, k_, v_, out_, lse_, dO, mask, record);
         }
         if (record) {
-            auto node = std::make_shared<SecondOrderNode>();
+            auto node = make_node<SecondOrderNode>();
             node->set_next_edges(torch::autograd::collect_next_edges(q_, k_, v_, dO));
             node->mask = mask;
             node->q = SavedVariable(q_, false); node->k = SavedVariable(k_, false); node->v = SavedVariable(v_, false);
@@ -238,7 +242,7 @@ Tensor sdpa(const Tensor& q, const Tensor& k, const Tensor& v, const Mask& m) {
         r = run_forward(q, k, v, m);
     }
     if (record) {
-        auto node = std::make_shared<SdpaNode>();
+        auto node = make_node<SdpaNode>();
         node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
         node->mask = m;
         node->q = SavedVariable(q, false); node->k = SavedVariable(k, false); node->v = SavedVariable(v, false);

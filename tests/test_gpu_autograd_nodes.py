@@ -56,3 +56,13 @@ def test_a_forward_mode_tangent_of_the_output_gradient_is_refused_where_a_graph_
         weight = fwAD.make_dual(dO.detach(), torch.ones_like(dO))
         with pytest.raises(NotImplementedError):
             torch.autograd.grad((out * weight).sum(), leaves, create_graph=True)
+
+
+def test_a_long_chain_of_calls_is_freed_without_recursion():
+    q, k, v = (torch.randn(1, 1, 1, 32, device="cuda").to(BF16) for _ in range(3))
+    out = q.requires_grad_(True)
+    for _ in range(200_000):
+        out = bob.sdpa_bob(out, k, v)
+    del out                                     # with a stack frame for each call this would overflow the stack
+    out = bob.sdpa_bob(q, k, v)
+    assert torch.equal(torch.autograd.grad(out.sum(), q)[0], torch.zeros_like(q))      # one key: no dependence on q
