@@ -256,12 +256,13 @@ static void set_strided(const void*& dst, long long& sb, long long& sh, long lon
 }
 
 // ---- forward with a few query rows ------------------------------------------------------------------
-// Up to kDecodeRows query rows per head go to decode_kernel whatever the number of keys: the sweep kernel would
-// do the work of 128 rows for them.  Where the caller's workspace is sized for it (BOB_SM100_SPLIT_KEYS), a head's keys
-// are divided until kDecodeCtas CTAs are there (two are resident per SM), but not below one round of a CTA's warps.
-// (The number is B200's and not asked of the device, so that the workspace's size depends on the geometry alone.)
-constexpr int kDecodeCtas = 4 * 148;
+// decode_kernel divides a head's keys until kDecodeCtas CTAs are there (two are resident per SM), but not below one
+// round of a CTA's warps.  (The numbers are B200's and not asked of the device, so that the workspace's size
+// depends on the geometry alone.)
+constexpr int kSms = 148, kDecodeCtas = 4 * kSms;
 struct DecodePlan { int k_lo, k_hi, splits, split_keys; size_t acc_offset, bytes; };     // offsets in the workspace
+
+static int decode_dpad(const bob_sm100_geom* g) { return g->D <= 32 ? 32 : (g->D <= 64 ? 64 : 128); }
 
 static DecodePlan decode_plan(const bob_sm100_geom* g) {
     DecodePlan d = {};
@@ -274,11 +275,9 @@ static DecodePlan decode_plan(const bob_sm100_geom* g) {
     }
     if (hi < lo) hi = lo = 0;
     d.k_lo = (int)lo; d.k_hi = (int)hi;
-    const int dpad = g->D <= 32 ? 32 : (g->D <= 64 ? 64 : 128);
-    const int64_t round = decode_round(dpad, g->Nq), rounds = std::max<int64_t>(1, (hi - lo + round - 1) / round);
+    const int64_t round = decode_round(decode_dpad(g), g->Nq), rounds = std::max<int64_t>(1, (hi - lo + round - 1) / round);
     const int64_t heads = (int64_t)g->B * g->Hq;
-    const int64_t want = !(g->flags & BOB_SM100_SPLIT_KEYS) ? 1
-                                                            : std::min<int64_t>({kDecodeMaxSplits, rounds, std::max<int64_t>(1, kDecodeCtas / heads)});
+    const int64_t want = std::min<int64_t>({kDecodeMaxSplits, rounds, std::max<int64_t>(1, kDecodeCtas / heads)});
     const int64_t per = (rounds + want - 1) / want;
     d.split_keys = (int)(per * round);
     d.splits = (int)((rounds + per - 1) / per);
@@ -290,6 +289,23 @@ static DecodePlan decode_plan(const bob_sm100_geom* g) {
         d.bytes = d.acc_offset + rows * g->D * sizeof(float);
     }
     return d;
+}
+
+// Whether a forward goes to decode_kernel.  The sweep kernel does the work of 128 rows for a few, but on the tensor cores
+// and the special-function unit, and its time grows with the rounds of one CTA per head; decode_kernel's arithmetic grows
+// with rows x heads x keys.  Measured, us, decode / sweep kernel, bf16, 4096 keys unless given:
+//   one row     128 heads D=64 31.9 / 39.0, D=128 51.4 / 53.4, 512 keys 17.4 / 16.5; 1024 heads D=64 166 / 219; 2 heads 10 / 37
+//   four rows   heads x D up to 4096 per round of 148 heads: 64 heads D=64 35 / 38, 32 heads D=128 37 / 47, 160 heads D=32 41 / 68
+//               beyond: 96 heads D=64 47 / 38, 64 heads D=128 57 / 49, 148 heads D=128 103 / 56, 512 keys 27 / 17
+//               keys for one round of a CTA's warps: 128 heads 64 keys D=128 6 / 12, 1024 heads 24 / 39
+// (two and three rows as four).  Without divided keys, which need a workspace of their size (BOB_SM100_SPLIT_KEYS), the
+// sweep kernel reads a long head faster.
+static bool takes_decode(const bob_sm100_geom* g) {
+    if (g->Nq > kDecodeRows) return false;
+    const DecodePlan d = decode_plan(g);
+    if (d.splits > 1 && !(g->flags & BOB_SM100_SPLIT_KEYS)) return false;
+    const int64_t heads = (int64_t)g->B * g->Hq;
+    return g->Nq == 1 || d.k_hi - d.k_lo <= decode_round(decode_dpad(g), g->Nq) || heads * decode_dpad(g) <= 4096 * ((heads + kSms - 1) / kSms);
 }
 
 template <bool BF16>
@@ -381,7 +397,7 @@ extern "C" size_t bob_sm100_workspace_bytes(int stage, const bob_sm100_geom* g) 
     if (!g || g->B <= 0 || g->Hq <= 0 || g->Hkv <= 0 || g->Nq <= 0 || g->Nk <= 0) return 0;
     size_t bytes = kStatusBlock;
     if (stage == BOB_SM100_STAGE_BWD2) bytes = bwd2_workspace_bytes(g);
-    if (stage == BOB_SM100_STAGE_FWD && g->Nq <= kDecodeRows) bytes = decode_plan(g).bytes;
+    if (stage == BOB_SM100_STAGE_FWD && takes_decode(g)) bytes = decode_plan(g).bytes;
     return bytes;
 }
 
@@ -424,7 +440,7 @@ extern "C" int bob_sm100_fwd(const bob_sm100_geom* g, const void* q, const void*
     if (!guard.ok) return kErrDevice;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int* sticky = sticky_word(g->device, true);
-    if (g->Nq <= kDecodeRows) return run_decode(g, q, k, v, out, lse, workspace, s);
+    if (takes_decode(g)) return run_decode(g, q, k, v, out, lse, workspace, s);
     if ((rc = begin_call(workspace, s))) return rc;
 
     SweepParams p;

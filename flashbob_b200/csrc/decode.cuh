@@ -16,7 +16,7 @@
 
 namespace bob {
 
-constexpr int kDecodeRows = 4;          // most query rows per head
+constexpr int kDecodeRows = 4;          // most query rows per head (which calls come here: takes_decode)
 constexpr int kDecodeThreads = 256;
 constexpr int kDecodeMaxSplits = 64;
 

@@ -55,8 +55,8 @@ enum { BOB_SM100_FP16 = 0, BOB_SM100_BF16 = 1 };
 enum { BOB_SM100_STAGE_FWD = 0, BOB_SM100_STAGE_BWD1 = 1, BOB_SM100_STAGE_BWD2 = 2 };
 /* geom->flags: the forward's workspace is as large as bob_sm100_workspace_bytes says for this very geometry (sizes,
  * mask and offsets), so a forward with at most four query rows may divide a head's keys between several CTAs and
- * park their parts there.  Without it the forward's workspace is 256 bytes for every geometry, and one CTA reads all
- * keys of a head of such a call. */
+ * park their parts there.  Without it the forward's workspace is 256 bytes for every geometry, and such a call goes
+ * through the kernel for many rows wherever keys would be divided. */
 enum { BOB_SM100_SPLIT_KEYS = 1 };
 
 typedef struct bob_sm100_geom {

@@ -53,6 +53,7 @@ def test_forward_stays_inside_its_workspace(flags, Nq, D):
     assert rc == 0 and lib.bob_sm100_read_status(ptr(ws), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
     assert (ws[size:] == 0x5a).all()
     s = q.double() @ k.double().transpose(2, 3) / math.sqrt(D)
-    # rounded to bf16 once: 2^-8 of a value
-    torch.testing.assert_close(out.double(), torch.softmax(s, -1) @ v.double(), rtol=1.05 * 2.0 ** -8, atol=2e-5)
+    # fp32 throughout and rounded to bf16 once, 2^-8 of a value; without the flag the kernel for many rows also rounds each
+    # probability p to bf16, which moves a result by at most 2^-8 sum(p |v|) <= 2^-8 * 0.8 and in fact by far less: 1e-3
+    torch.testing.assert_close(out.double(), torch.softmax(s, -1) @ v.double(), rtol=1.05 * 2.0 ** -8, atol=2e-5 if flags else 1e-3)
     torch.testing.assert_close(lse.double(), torch.logsumexp(s, -1), rtol=2e-5, atol=2e-5)

@@ -1,4 +1,4 @@
-"""Forward with a few query rows: infinite scores, against fp64 attention."""
+"""Forward with a few query rows: infinite scores, and both sides of the line between its two kernels, against fp64 attention."""
 
 import math
 
@@ -29,3 +29,21 @@ def test_an_infinite_score_makes_its_row_nan_and_no_other(Nq, Nk, entry, width):
         s[..., 33] = -math.inf
         # the probabilities of the sweep kernel and every result are rounded to bf16: 2^-8 of a value, or of the sum's scale
         torch.testing.assert_close(out[:, :, 1::2].double(), torch.softmax(s, -1) @ v.double(), rtol=2.0 ** -7, atol=4e-3)
+
+
+@pytest.mark.parametrize("heads,D,Nk", [
+    (32, 128, 200), (33, 128, 200), (64, 64, 300), (65, 64, 300), (128, 32, 600), (129, 32, 600),     # heads x D of a round
+    (149, 32, 600), (148, 128, 65), (149, 48, 200),                                                   # ... of two rounds
+    (200, 128, 64), (200, 128, 65), (200, 64, 128), (200, 64, 129), (200, 32, 256), (200, 32, 257),   # one round of keys
+])
+@pytest.mark.parametrize("Nq", [2, 4])
+def test_both_sides_of_the_line_between_the_kernels(heads, D, Nk, Nq):
+    gen = torch.Generator().manual_seed(6)
+    q, k, v = (torch.randn(1, heads, n, D, generator=gen).to(torch.bfloat16).cuda() for n in (Nq, Nk, Nk))
+    out, lse = ops.attention_forward(q, k, v, is_causal=True, window_size=0, q_offset=Nk - Nq, k_offset=0, scale=None)
+    s = q.double() @ k.double().transpose(2, 3) / math.sqrt(D)
+    s = s.masked_fill(torch.ones(Nq, Nk, dtype=torch.bool, device="cuda").triu(Nk - Nq + 1), -math.inf)
+    # results are rounded once, by up to 2^-9 of a value (bf16); the kernel for many rows rounds each probability likewise,
+    # which moves a result by about 2^-9 sqrt(sum p^2 v^2) < 2^-9 * 0.5: five of that
+    torch.testing.assert_close(out.double(), torch.softmax(s, -1) @ v.double(), rtol=2.0 ** -8, atol=5e-3)
+    torch.testing.assert_close(lse.double(), torch.logsumexp(s, -1), rtol=2e-5, atol=2e-5)
