@@ -1,4 +1,7 @@
-"""What the operator's autograd nodes owe to the rest of PyTorch's autograd."""
+"""What the operator's autograd nodes owe to the rest of PyTorch's autograd: tracing, forward mode, saved-tensor hooks,
+checkpointing, batched gradients, release, streams and threads."""
+
+import threading
 
 import pytest
 import torch
@@ -66,3 +69,85 @@ def test_a_long_chain_of_calls_is_freed_without_recursion():
     del out                                     # with a stack frame for each call this would overflow the stack
     out = bob.sdpa_bob(q, k, v)
     assert torch.equal(torch.autograd.grad(out.sum(), q)[0], torch.zeros_like(q))      # one key: no dependence on q
+
+
+def test_saved_tensor_hooks_see_and_replace_the_saved_tensors():
+    leaves, dO, bars = _inputs(0)
+    want = _step(causal, leaves, dO, bars)
+    packed = []
+
+    def pack(t):
+        packed.append(tuple(t.shape))
+        return t.cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        _same(_step(causal, leaves, dO, bars), want)
+    # forward: q, k, v, out, lse; first backward kept in the graph: q, k, v, dO, out, lse, dQ, delta, pk
+    assert len(packed) == 5 + 9
+
+
+@pytest.mark.parametrize("reentrant", [False, True])
+def test_checkpointed_call_gives_the_same_gradients(reentrant):
+    leaves, dO, _ = _inputs(0)
+    want = torch.autograd.grad(causal(*leaves), leaves, dO.detach())
+    again = [t.detach().requires_grad_(True) for t in leaves]
+    out = torch.utils.checkpoint.checkpoint(causal, *again, use_reentrant=reentrant)
+    out.backward(dO.detach())
+    _same([t.grad for t in again], want)
+
+
+def test_batched_gradients_are_refused_with_an_error():
+    leaves, dO, _ = _inputs(0)
+    out = causal(*leaves)
+    batch = torch.stack([dO.detach()] * 2)
+    for keep in (False, True):
+        with pytest.raises(RuntimeError):
+            torch.autograd.grad(out, leaves, batch, retain_graph=True, create_graph=keep, is_grads_batched=True)
+
+
+def test_a_released_graph_is_refused_and_a_retained_one_repeats():
+    leaves, dO, bars = _inputs(0)
+    out = causal(*leaves)
+    a = torch.autograd.grad(out, leaves, dO, retain_graph=True)
+    _same(torch.autograd.grad(out, leaves, dO), a)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out, leaves, dO)
+    out = causal(*leaves)
+    first = torch.autograd.grad(out, leaves, dO, create_graph=True)
+    a = torch.autograd.grad(first, leaves, bars, retain_graph=True)
+    _same(torch.autograd.grad(first, leaves, bars), a)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(first, leaves, bars)
+
+
+def test_an_input_changed_in_place_is_noticed():
+    leaves, dO, _ = _inputs(0)
+    mid = leaves[0] * 1
+    out = causal(mid, *leaves[1:])
+    mid.add_(1)
+    with pytest.raises(RuntimeError, match="inplace operation"):
+        torch.autograd.grad(out, leaves, dO)
+
+
+@pytest.mark.parametrize("nq", [48, 1])
+def test_steps_on_other_streams_and_threads_give_the_same_bits(nq):
+    cases = [_inputs(s, nq, 700) for s in range(4)]
+    want = [_step(causal, *c) for c in cases]
+    torch.cuda.synchronize()
+    got, errors = [None] * 4, []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(20):
+                    got[i] = _step(causal, *cases[i])
+            torch.cuda.synchronize()
+        except Exception as e:                  # seen by the main thread below
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors, errors
+    for g, w in zip(got, want):
+        _same(g, w)

@@ -15,7 +15,15 @@ BF16, FP16 = torch.bfloat16, torch.float16
 @pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D,dtype,mask,order", [
     (1, 2, 2, 1, 1, 64, BF16, {}, "bhnd"),
     (1, 2, 2, 1, 16384, 64, BF16, {}, "bhnd"),                      # 64 splits of a head
-    (2, 3, 3, 1, 257, 32, FP16, {}, "bnhd"),                        # one key past a round
+    (2, 3, 3, 1, 257, 32, FP16, {}, "bnhd"),                        # half a round
+    (2, 3, 3, 1, 513, 32, FP16, {}, "bnhd"),                        # one key past a round: two CTAs, the last with one key
+    (2, 3, 3, 1, 257, 64, FP16, {}, "bhnd"),
+    (2, 3, 3, 1, 129, 128, BF16, {}, "bnhd"),
+    (2, 3, 3, 4, 257, 32, BF16, {}, "bhnd"),                        # (more than one row: rounds half as long)
+    (1, 3, 3, 3, 129, 64, BF16, {}, "bnhd"),
+    (1, 3, 3, 2, 65, 128, FP16, {}, "bhnd"),
+    (1, 2, 2, 1, 5000, 32, BF16, {}, "bhnd"),                       # many parts at head dim 32
+    (1, 2, 2, 4, 5000, 32, BF16, {}, "bnhd"),
     (1, 5, 5, 1, 1023, 128, BF16, {}, "bnhd"),
     (3, 200, 200, 1, 129, 64, FP16, {}, "bhnd"),                    # more heads than CTAs wanted: no split
     (2, 4, 4, 4, 2048, 64, BF16, dict(is_causal=True), "bnhd"),     # right-aligned rectangle

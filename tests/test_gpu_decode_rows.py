@@ -1,4 +1,5 @@
-"""Forward with a few query rows: infinite scores, and both sides of the line between its two kernels, against fp64 attention."""
+"""Forward with a few query rows: infinite scores and both sides of the line between its two kernels, against fp64 attention;
+the same bits from repeats, graph replays and concurrent streams."""
 
 import math
 
@@ -47,3 +48,39 @@ def test_both_sides_of_the_line_between_the_kernels(heads, D, Nk, Nq):
     # which moves a result by about 2^-9 sqrt(sum p^2 v^2) < 2^-9 * 0.5: five of that
     torch.testing.assert_close(out.double(), torch.softmax(s, -1) @ v.double(), rtol=2.0 ** -8, atol=5e-3)
     torch.testing.assert_close(lse.double(), torch.logsumexp(s, -1), rtol=2e-5, atol=2e-5)
+
+
+def _wide(seed, heads=3, Nq=1, Nk=9000, D=64):
+    gen = torch.Generator().manual_seed(seed)
+    return tuple(torch.randn(2, heads, n, D, generator=gen).to(torch.bfloat16).cuda() for n in (Nq, Nk, Nk))
+
+
+_FULL = dict(is_causal=False, window_size=0, q_offset=0, k_offset=0, scale=None)
+
+
+@pytest.mark.parametrize("Nq,D", [(1, 64), (1, 32), (4, 64), (3, 128)])
+def test_divided_heads_repeat_bit_for_bit_in_eager_calls_replays_and_streams(Nq, D, monkeypatch):
+    """Which CTA of a head finishes last, and adds the parts, differs from run to run; their order does not."""
+    monkeypatch.setattr(ops, "_CHECK_STATUS", False)         # reading the status waits, which a capture does not allow
+    cases = [_wide(s, Nq=Nq, D=D) for s in range(4)]
+    want = [ops.attention_forward(*c, **_FULL) for c in cases]
+    same = lambda got, i: torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1])
+    for _ in range(50):
+        assert same(ops.attention_forward(*cases[0], **_FULL), 0)
+    graph = torch.cuda.CUDAGraph()
+    static = tuple(t.clone() for t in cases[0])
+    with torch.cuda.graph(graph):
+        got = ops.attention_forward(*static, **_FULL)
+    for i in (0, 1, 2, 3, 0):
+        for s, t in zip(static, cases[i]):
+            s.copy_(t)
+        graph.replay()
+        assert same(got, i)
+    torch.cuda.synchronize()
+    streams, results = [torch.cuda.Stream() for _ in cases], []
+    for _ in range(20):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                results.append((i, ops.attention_forward(*cases[i], **_FULL)))
+    torch.cuda.synchronize()
+    assert all(same(got, i) for i, got in results)
