@@ -15,11 +15,11 @@
 // holds column j of the score matrix and the operands come out already transposed; the per-query
 // statistics then vary along the tensor-memory columns and are staged in shared memory.
 //
-// Warp roles: NG groups of 128*NSPLIT pointwise threads, one MMA warp (warp-uniform control flow, one
-// elected lane issues) and one TMA warp.  Tiles of the other side sit in a ring of 2 to 6 stages;
-// the scores of tile t+1 are issued before the output products of tile t, so the tensor pipe works
-// while the pointwise threads convert tile t.  Work items (own tile x head x batch) are handed out
-// longest first, either from a global counter (persistent launches) or one per CTA.
+// Warp roles: NG groups of 128*NSPLIT pointwise threads, and four role warps - a TMA warp, two that issue products (one
+// the scores, as far ahead as accumulators are free, one the outputs, as operands arrive; a single elected thread
+// runs the loop of each) and one that moves results.  Tiles of the other side sit in a ring of 2 to 8 tiles.  Work
+// items (own tile x head x batch) are handed out longest first, either from a global counter (persistent launches) or
+// one per CTA.
 //
 // The algebra follows the reference's second backward (reference: src/bob/kernels/common.py:15-30
 // for the formulas, :463-654 for the row-owned tile body and epilogue, :661-786 for the
@@ -55,7 +55,7 @@ struct SweepParams {
     // geometry
     int B, Hq, Hkv, G, Nq, Nk, D;
     int is_causal, window;
-    int delta_off;                // q_offset - k_offset, clamped to +-2^30
+    int delta_off;                // q_offset - k_offset, clamped to +-2^29
     float scale;
     int has_uq, has_uk, has_uv;   // 0 = that tangent is undefined (treated as zero, products skipped)
     // global tensors read with plain loads (element strides: batch, head, row; unit head-dim stride)
@@ -72,7 +72,6 @@ struct SweepParams {
     // results, contiguous [B, H, N, D] in the input dtype
     void* res0;
     void* res1;
-    void* res2;
     int* status;
     int* sticky;                  // optional second word that a CTA giving up also writes (host-visible memory)
     int* work_counter;            // persistent launches: next work item (zeroed by the host); null: one item per CTA
@@ -182,7 +181,10 @@ struct SweepConfig {
     // around in registers, so that a warp-wide access touches 4 lines.  With a row per lane it touches 32, and the
     // row-owned second backward spent 19600 cycles between an item's last tile and the end of its epilogue (a tile
     // takes 1900), the column-owned one 7100, the first backward 9400; with the rows turned around 13900, 5000 and 6900
-    // (kernels at H=32 S=2048: 184 to 174, 167 to 165 and 88 to 83 us).
+    // (kernels at H=32 S=2048: 184 to 174, 167 to 165 and 88 to 83 us).  The price is paid where an item has half a tile of
+    // rows or less and so had few lines to touch: the second backward's two kernels over one such item per CTA take 14.4
+    // and 12.2 us, against 12.4 and 10.4 with a row per lane (a full tile: 16.5 and 14.4 against 20.7 and 16.4).  Leaving out the
+    // turns of warps without rows did not help (14.4), and slowed full tiles (18.4).
     static constexpr bool TURN_IO = BWD2 && DPAD == 128;
     static constexpr bool TURN_PK = MODE == kBwd1Row && !STAGED_PK;
     static_assert(!TURN_IO || DPAD / (NSPLIT * NG) == 64, "128 bytes of a 16-bit row per thread");
@@ -316,7 +318,7 @@ sweep_kernel(const __grid_constant__ SweepParams p) {
     const int per_rank = grid_heads * p.B;
     const int n_items = n_own_tiles * per_rank;
     const int n_outer = COL ? p.G : 1;
-    const int doff = p.delta_off;                // q_offset - k_offset, within +-2^29 (see the host's fill_common)
+    const int doff = p.delta_off;                // q_offset - k_offset, within +-2^29 (see the host's fill_mask)
     // kernel parameters that the per-tile code needs, read once
     const bool causal = p.is_causal != 0;
     const int window = p.window;
